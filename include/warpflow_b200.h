@@ -327,6 +327,10 @@ typedef struct wf_stepper wf_stepper;
  * after its predecessor finished, which frees SMs for other streams when
  * many steppers run concurrently (ensembles, serving). */
 #define WF_STEP_SERIAL 2
+/* With WF_STEP_SERIAL: the half-sweeps of the multigrid still launch with
+ * programmatic dependent launch (each computes its indices and reads its
+ * right-hand side while the one before it runs). */
+#define WF_STEP_CHAIN 8
 WF_API int wf_stepper_create(const wf_case* c, int32_t mode, wf_stepper** out);
 /* One FlowSolver.step(): enqueue the step on `stream`.  No host sync. */
 WF_API int wf_stepper_step(wf_stepper* s, void* stream);
@@ -340,7 +344,7 @@ WF_API int wf_stepper_destroy(wf_stepper* s);
  * every case's step (as wf_stepper_create builds it) to a single CUDA graph
  * as independent branches, so the device schedules all cases' kernels
  * concurrently without a stream per case.  `cases` are copied; mode 0 or
- * WF_STEP_SERIAL, optionally | WF_ENS_BUCKETS: cases of the same size and
+ * WF_STEP_SERIAL (with WF_STEP_CHAIN or without), optionally | WF_ENS_BUCKETS: cases of the same size and
  * numerics (any Re and lid velocity; the same shared coarse operator) then
  * form buckets, and each bucket is ONE branch whose every kernel launch
  * serves all its cases (grids stacked along z, a device table of the cases'

@@ -25,6 +25,16 @@ __device__ __forceinline__ void pdl_entry() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
+// The other order, for chains of short dependent kernels: a kernel lets its
+// successor launch only after its own wait, so whatever the successor does
+// ahead of its wait runs when every kernel before its predecessor has
+// completed.  Data those wrote may therefore be read ahead of the wait
+// (__ldcg: past the L1, which may hold lines of an earlier pass).
+__device__ __forceinline__ void pdl_chain() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // ---- bucket batching (see Batch in wf_internal.h) -------------------------
 // the case of this block, its z index within the case's grid, the case's z
 // extent; a case's buffers

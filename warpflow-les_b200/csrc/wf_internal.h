@@ -40,8 +40,9 @@ extern thread_local long g_launches;
 
 inline int64_t padded(int n) { return (int64_t)n + 2 * NPL; }
 
-// programmatic dependent launch on (default) or off (WF_PDL=0)
-bool pdl_enabled();
+// programmatic dependent launch on (default) or off (WF_PDL=0, WF_STEP_SERIAL);
+// chain: for the half-sweeps, which WF_STEP_CHAIN keeps on
+bool pdl_enabled(bool chain = false);
 
 // one thread per cell of an ni x nj x nk box: CTAs of 32 (k) x 8 (j) threads,
 // grid z = i
@@ -96,7 +97,7 @@ constexpr bool takes_batch() {
 // attribute when enabled.  A kernel whose last parameter is a Batch gets the
 // calling thread's bucket (grid z multiplied by its case count); any other
 // kernel refuses to launch while a bucket is being built.
-template <typename... ExpTypes, typename... ActTypes>
+template <bool CHAIN = false, typename... ExpTypes, typename... ActTypes>
 inline cudaError_t launch_k(void (*kernel)(ExpTypes...), dim3 grid, dim3 block, size_t smem,
                             cudaStream_t s, ActTypes&&... args) {
   cudaLaunchConfig_t cfg = {};
@@ -106,7 +107,7 @@ inline cudaError_t launch_k(void (*kernel)(ExpTypes...), dim3 grid, dim3 block, 
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   int na = 0;
-  if (pdl_enabled()) {
+  if (pdl_enabled(CHAIN)) {
     at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[na].val.programmaticStreamSerializationAllowed = 1;
     ++na;
@@ -122,6 +123,13 @@ inline cudaError_t launch_k(void (*kernel)(ExpTypes...), dim3 grid, dim3 block, 
     if (bc.tab) return cudaErrorNotSupported;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<ActTypes&&>(args)...);
   }
+}
+
+// launch_k for the kernels of a half-sweep chain (pdl_chain)
+template <typename K, typename... ActTypes>
+inline cudaError_t launch_chain(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                ActTypes&&... args) {
+  return launch_k<true>(kernel, grid, block, smem, s, static_cast<ActTypes&&>(args)...);
 }
 
 int validate_case(const wf_case& c);
@@ -169,6 +177,7 @@ int launch_scalars_init(wf_scalars* sc, double dt0, double rrey, double ulid, cu
 // wf_set_launch_shape (the autotuner).
 constexpr int SHAPE_CONV = 0, SHAPE_SPLIT = 1;
 void launch_shape(int kind, int n, int* a, int* b, int* c);
+bool launch_shape_set(int kind, int n);   // wf_set_launch_shape set one for this size
 int set_launch_shape(int kind, int n, int a, int b, int c);
 
 // ---- multigrid -----------------------------------------------------------

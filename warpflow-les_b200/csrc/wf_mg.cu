@@ -32,6 +32,7 @@
 namespace wf {
 
 constexpr int MG_TPB = 256;
+constexpr int RBGS_TPB = 128;
 
 template <class T>
 struct Lvl {
@@ -128,33 +129,60 @@ static ApRecip<T> ap_recip(const Lvl<T>& L) {
 }
 
 // one colour half-sweep (multigrid.py:70-90): update where (i+j+k+color)%2==1
+// One thread per cell of the colour, the cells of a plane i numbered flat
+// (rnh = 1 / cells per row).  A launch of these small levels is a chain of
+// latencies (start, index arithmetic, one round of loads, the dependent FP64
+// operations, the store); everything that does not depend on the launch ahead
+// comes before the wait, and the quotient is the reciprocal form's.  us per
+// half-sweep in a graph, before / now: 32^3 1.87 / 1.19, 40^3 2.12 / 1.30,
+// 48^3 2.07 / 1.45.  pre: the level's rhs was complete before the launch ahead
+// of this one (pdl_chain), so it may be read ahead of the wait.
 template <class T>
-__global__ void __launch_bounds__(MG_TPB) k_rbgs(const Lvl<T> L0, int color, const Batch bt) {
-  pdl_entry();
-  if (bt_skip(bt)) return;
+__global__ void __launch_bounds__(RBGS_TPB) k_rbgs(const Lvl<T> L0, int color, int pre,
+                                                   const float rnh,
+                                                   const __grid_constant__ ApRecip<T> rt,
+                                                   const Batch bt) {
+  if (bt.tab) {
+    pdl_chain();
+    if (bt_skip(bt)) return;
+  }
   const Lvl<T> L = rebase(L0, bt);
   const int n = L.n;
   const int nh = (n + 1) >> 1;
-  {  // one thread per cell: x = kk (runs of 32), y = j (groups of 8), z = i
-    const int kx_ = blockIdx.x * 32 + threadIdx.x, jy_ = blockIdx.y * 8 + threadIdx.y;
-    if (kx_ >= nh || jy_ >= n) return;
-    const int kk = kx_;
-    const int j = jy_;
-    const int i = bt_z(bt);
-    const int k = 2 * kk + ((1 + i + j + color) & 1);
-    if (k >= n) return;
-    const long c = lid(L, i + 1, j + 1, k + 1);
-    const T aw = i > 0 ? L.ax : T(0), ae = i < n - 1 ? L.ax : T(0);
-    const T as = j > 0 ? L.ay : T(0), an = j < n - 1 ? L.ay : T(0);
-    const T ab = k > 0 ? L.az : T(0), at = k < n - 1 ? L.az : T(0);
-    const T ap = -(aw + ae + as + an + ab + at);
-    const T* phi = L.phi;
-    const T s = aw * phi[c - L.sI] + ae * phi[c + L.sI] + as * phi[c - L.sJ] +
-                an * phi[c + L.sJ] + ab * phi[c - 1] + at * phi[c + 1];
-    const T x = (L.rhs[c] - s) / ap;
-    L.phi[c] = x;
-    ring_mirror(L, i, j, k, c, x);
-  }
+  const int t = blockIdx.x * RBGS_TPB + threadIdx.x;
+  const int j = (int)(((float)t + 0.5f) * rnh);
+  const int i = bt_z(bt);
+  const int k = 2 * (t - j * nh) + ((1 + i + j + color) & 1);
+  const bool on = j < n && k < n;
+  const int sI = (int)L.sI, sJ = (int)L.sJ;
+  const long c = (long)(i + 1) * L.sI + (j + 1) * sJ + k + 1;
+  const T aw = i > 0 ? L.ax : T(0), ae = i < n - 1 ? L.ax : T(0);
+  const T as = j > 0 ? L.ay : T(0), an = j < n - 1 ? L.ay : T(0);
+  const T ab = k > 0 ? L.az : T(0), at = k < n - 1 ? L.az : T(0);
+  const T ap = -(aw + ae + as + an + ab + at);
+  const T y = rt.y[on ? 9 * ((i > 0) + (i < n - 1)) + 3 * ((j > 0) + (j < n - 1)) + (k > 0) +
+                            (k < n - 1)
+                      : 0];
+  T r = T(0);
+  if (pre && on) r = __ldcg(L.rhs + c);
+  if (!bt.tab) pdl_chain();
+  if (!on) return;
+  if (!pre) r = L.rhs[c];
+  const T* phi = L.phi + c;
+  const T s = aw * phi[-sI] + ae * phi[sI] + as * phi[-sJ] + an * phi[sJ] + ab * phi[-1] +
+              at * phi[1];
+  const T x = div_by_recip(r - s, ap, y);
+  L.phi[c] = x;
+  ring_mirror(L, i, j, k, c, x);
+}
+
+template <class T>
+static int launch_rbgs(const Lvl<T>& L, int color, bool pre, cudaStream_t s) {
+  const int nh = (L.n + 1) / 2;
+  WF_CK(launch_chain(k_rbgs<T>, dim3((L.n * nh + RBGS_TPB - 1) / RBGS_TPB, 1, L.n), RBGS_TPB, 0, s,
+                     L, color, pre ? 1 : 0, 1.0f / (float)nh, ap_recip(L)));
+  WF_CKL("k_rbgs");
+  return WF_OK;
 }
 
 // restriction (multigrid.py:93-119): rhs_c = 1/8 sum of the 8 fine residuals;
@@ -1637,10 +1665,7 @@ static int apply_coarse_op(const Lvl<T>& L, const T* op, T* part, cudaStream_t s
   WF_CKL("k_cop_gemm");
   WF_CK(launch_k(k_cop_out<T>, (P.M + 255) / 256, 256, 0, s, (const T*)Y, prod, P.nrep, L));
   WF_CKL("k_cop_out");
-  for (int color = 0; color < 2; ++color) {
-    WF_CK(launch_k(k_rbgs<T>, cells3(L.n, L.n, (L.n + 1) / 2), cell_block(), 0, s, L, color));
-    WF_CKL("k_rbgs");
-  }
+  for (int color = 0; color < 2; ++color) WF_TRY(launch_rbgs(L, color, color > 0, s));
   return WF_OK;
 }
 
@@ -1769,10 +1794,12 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
 // reads only the other colour and rhs, which it does not write.
 template <class T, int CPT>
 __global__ void __launch_bounds__(32 * SPLIT_ROWS)
-    k_rbgs_split(const Lvl<T> L0, T* sp, const T* sr, int color,
+    k_rbgs_split(const Lvl<T> L0, T* sp, const T* sr, int color, int pre,
                  const __grid_constant__ ApRecip<T> rt, const Batch bt) {
-  pdl_entry();
-  if (bt_skip(bt)) return;
+  if (bt.tab) {
+    pdl_chain();
+    if (bt_skip(bt)) return;
+  }
   const Lvl<T> L = rebase(L0, bt);
   if (bt.tab) {
     sp = L.tmp;
@@ -1782,7 +1809,7 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
   const int h0 = blockIdx.x * 32 * CPT + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int i = bt_z(bt);
-  if (j >= n || h0 >= nh) return;
+  const bool on = j < n && h0 < nh;
   const int H = (n + 2) >> 1, tI = (int)L.tI, tJ = (int)L.tJ;
   const int pr = (i + j + color) & 1;       // parity of a = k+1 of this row's colour
   const long r = (long)(i + 1) * L.tI + (long)(j + 1) * L.tJ;
@@ -1793,6 +1820,13 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
   const T as = j > 0 ? L.ay : T(0), an = j < n - 1 ? L.ay : T(0);
   const int pij = 9 * ((i > 0) + (i < n - 1)) + 3 * ((j > 0) + (j < n - 1));
   T vw[CPT], ve[CPT], vs[CPT], vn[CPT], vb[CPT], vt[CPT], vr[CPT];
+  if (pre && on) {
+#pragma unroll
+    for (int u = 0; u < CPT; ++u)
+      if (u == 0 || h0 + 32 * u < nh) vr[u] = __ldcg(rr + 32 * u);
+  }
+  if (!bt.tab) pdl_chain();
+  if (!on) return;
 #pragma unroll
   for (int u = 0; u < CPT; ++u) {
     if (u == 0 || h0 + 32 * u < nh) {
@@ -1802,7 +1836,7 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
       vn[u] = own[32 * u + tJ];
       vb[u] = oth[32 * u];
       vt[u] = oth[32 * u + 1];
-      vr[u] = rr[32 * u];
+      if (!pre) vr[u] = rr[32 * u];
     }
   }
 #pragma unroll
@@ -1814,6 +1848,71 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
       const T s = aw * vw[u] + ae * ve[u] + as * vs[u] + an * vn[u] + ab * vb[u] + at * vt[u];
       own[32 * u] = div_by_recip(vr[u] - s, ap, rt.y[pij + (k > 0) + (k < n - 1)]);
     }
+  }
+}
+
+// the same half-sweep with the colour's cells of a plane numbered flat
+// (rnh = 1 / cells per half-row), CPT cells a thread
+constexpr int FLAT_MAX_N = 104;
+
+template <class T, int CPT>
+__global__ void __launch_bounds__(MG_TPB)
+    k_rbgs_flat(const Lvl<T> L0, T* sp, const T* sr, int color, int pre, const float rnh,
+                const __grid_constant__ ApRecip<T> rt, const Batch bt) {
+  if (bt.tab) {
+    pdl_chain();
+    if (bt_skip(bt)) return;
+  }
+  const Lvl<T> L = rebase(L0, bt);
+  if (bt.tab) {
+    sp = L.tmp;
+    sr = L.tmp + (long)(L.n + 2) * (L.n + 2) * (L.n + 2);
+  }
+  const int n = L.n, nh = n >> 1;
+  const int i = bt_z(bt);
+  const int H = (n + 2) >> 1, tI = (int)L.tI, tJ = (int)L.tJ;
+  const T aw = i > 0 ? L.ax : T(0), ae = i < n - 1 ? L.ax : T(0);
+  const int pi = 9 * ((i > 0) + (i < n - 1));
+  sp += (long)(i + 1) * L.tI;
+  sr += (long)(i + 1) * L.tI;
+  int own[CPT], oth[CPT], jj[CPT], kk[CPT];
+  T x[CPT];
+#pragma unroll
+  for (int u = 0; u < CPT; ++u) {
+    const int t = (blockIdx.x * CPT + u) * MG_TPB + threadIdx.x;
+    const int j = (int)(((float)t + 0.5f) * rnh), h = t - j * nh;
+    const int pr = (i + j + color) & 1;
+    jj[u] = j;
+    kk[u] = 2 * h + 1 - pr;
+    own[u] = (j + 1) * tJ + pr * H + 1 - pr + h;
+    oth[u] = (j + 1) * tJ + (1 - pr) * H + h;
+    x[u] = T(0);
+    if (pre && j < n) x[u] = __ldcg(sr + own[u]);
+  }
+  if (!bt.tab) pdl_chain();
+  T vw[CPT], ve[CPT], vs[CPT], vn[CPT], vb[CPT], vt[CPT];
+#pragma unroll
+  for (int u = 0; u < CPT; ++u) {
+    if (jj[u] >= n) continue;
+    const T* p = sp + own[u];
+    vw[u] = p[-tI];
+    ve[u] = p[tI];
+    vs[u] = p[-tJ];
+    vn[u] = p[tJ];
+    vb[u] = sp[oth[u]];
+    vt[u] = sp[oth[u] + 1];
+    if (!pre) x[u] = sr[own[u]];
+  }
+#pragma unroll
+  for (int u = 0; u < CPT; ++u) {
+    const int j = jj[u], k = kk[u];
+    if (j >= n) continue;
+    const T as = j > 0 ? L.ay : T(0), an = j < n - 1 ? L.ay : T(0);
+    const T ab = k > 0 ? L.az : T(0), at = k < n - 1 ? L.az : T(0);
+    const T ap = -(aw + ae + as + an + ab + at);
+    const T y = rt.y[pi + 3 * ((j > 0) + (j < n - 1)) + (k > 0) + (k < n - 1)];
+    const T s = aw * vw[u] + ae * ve[u] + as * vs[u] + an * vn[u] + ab * vb[u] + at * vt[u];
+    sp[own[u]] = div_by_recip(x[u] - s, ap, y);
   }
 }
 
@@ -1851,15 +1950,16 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
 }
 
 // smallest even level edge that relaxes on the split copy (WF_SPLIT_MIN
-// overrides both): 80 for FP64, 128 for FP32, whose 80^3 level stays in L2
-// (step time at 80^3, FP64 1.332 ms split vs 1.348 in place; mixed 1.255 vs 1.184)
-static int split_min_n(bool fp32) {
+// overrides it).  us per step, split from 128 / 80 / 48: 80^3 mixed 782 / 707 /
+// 705, 96^3 mixed 1091 / 906 / 933; FP64 half-sweep at 64^3 2.07 in place,
+// 1.68 split, at 48^3 1.47 and 1.36, less than the copies cost there
+static int split_min_n() {
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("WF_SPLIT_MIN");
     v = e ? atoi(e) : 0;
   }
-  return v > 0 ? v : (fp32 ? 128 : 80);
+  return v > 0 ? v : 64;
 }
 
 // level -> split copies (phi, and rhs unless the scratch already holds it)
@@ -1874,25 +1974,39 @@ static int split_in(const Lvl<T>& L, bool with_rhs, cudaStream_t s) {
   return WF_OK;
 }
 
-// the half-sweeps of a relax on the split copies
+// the half-sweeps of a relax on the split copies.  A half-row of a level below
+// 104 cells does not fill k_rbgs_split's warps (40 of 64 or 128 lanes at 80^3)
+// and its CTAs are many and small: there the cells are numbered flat, one per
+// thread, two from 86 (the CTAs of one colour are then about one wave).  us per
+// half-sweep in a graph, rows / flat x 1 / flat x 2, FP64: 64^3 2.10 / 1.68 /
+// 1.86, 72^3 2.74 / 2.12 / 2.14, 80^3 2.91 / 2.09 / 2.14, 88^3 3.61 / 2.85 /
+// 2.89, 96^3 4.00 / 3.24 / 3.02, 104^3 3.58 / 3.93 / 3.59, 128^3 4.82 / 6.27 /
+// 5.64.  A shape set for the level (wf_set_launch_shape) takes the rows form.
 template <class T>
 static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
-  const int m = L.n + 2;
+  const int m = L.n + 2, nh = L.n / 2;
   T* sp = L.tmp;
   const T* sr = L.tmp + (long)m * m * m;
+  const ApRecip<T> rt = ap_recip(L);
+  const bool flat = L.n < FLAT_MAX_N && !launch_shape_set(SHAPE_SPLIT, L.n);
+  const int cells = L.n > 84 ? 2 : 1;
   int cpt, rows, one;
   launch_shape(SHAPE_SPLIT, L.n, &cpt, &rows, &one);   // cpt in {1, 2, 4, 8}, rows <= SPLIT_ROWS
-  const dim3 grid((L.n / 2 + 32 * cpt - 1) / (32 * cpt), (L.n + rows - 1) / rows, L.n);
-  const ApRecip<T> rt = ap_recip(L);
+  const dim3 grid((nh + 32 * cpt - 1) / (32 * cpt), (L.n + rows - 1) / rows, L.n);
+  const dim3 fgrid((L.n * nh + MG_TPB * cells - 1) / (MG_TPB * cells), 1, L.n);
   auto kern = cpt == 8   ? k_rbgs_split<T, 8>
               : cpt == 4 ? k_rbgs_split<T, 4>
               : cpt == 2 ? k_rbgs_split<T, 2>
                          : k_rbgs_split<T, 1>;
-  for (int it = 0; it < nsweeps; ++it) {
-    for (int color = 0; color < 2; ++color) {
-      WF_CK(launch_k(kern, grid, dim3(32, rows), 0, s, L, sp, sr, color, rt));
-      WF_CKL("k_rbgs_split");
-    }
+  auto kflat = cells == 2 ? k_rbgs_flat<T, 2> : k_rbgs_flat<T, 1>;
+  for (int h = 0; h < 2 * nsweeps; ++h) {
+    // from the second half-sweep on, the launch ahead is a half-sweep
+    const int pre = h > 0 ? 1 : 0;
+    if (flat)
+      WF_CK(launch_chain(kflat, fgrid, MG_TPB, 0, s, L, sp, sr, h & 1, pre, 1.0f / (float)nh, rt));
+    else
+      WF_CK(launch_chain(kern, grid, dim3(32, rows), 0, s, L, sp, sr, h & 1, pre, rt));
+    WF_CKL("k_rbgs_split");
   }
   return WF_OK;
 }
@@ -2368,7 +2482,7 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
     if (nsweeps > 12 && strat == 1 && try_coarse_cluster<T>(L, nsweeps, s, &rc)) return rc;
     if (try_coarse<T>(L, nsweeps, s, &rc)) return rc;
   }
-  if (L.tmp && (L.n & 1) == 0 && L.n >= split_min_n(sizeof(T) == 4))
+  if (L.tmp && (L.n & 1) == 0 && L.n >= split_min_n())
     return relax_split<T>(L, nsweeps, rhs_ready, s);
   if (!bucket) {
     int rc = WF_OK;
@@ -2383,12 +2497,8 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
       WF_TRY(launch_sweep2<T>(L.tmp, L.tI, L.tJ, L.phi, L.sI, L.sJ, L, ring, s));
     }
     if (nsweeps & 1) {
-      const long half = (long)L.n * L.n * ((L.n + 1) / 2);
-      const int nb = mg_blocks(half);
-      WF_CK(launch_k(k_rbgs<T>, cells3(L.n, L.n, (L.n + 1) / 2), cell_block(), 0, s, L, 0));
-      WF_CKL("k_rbgs");
-      WF_CK(launch_k(k_rbgs<T>, cells3(L.n, L.n, (L.n + 1) / 2), cell_block(), 0, s, L, 1));
-      WF_CKL("k_rbgs");
+      WF_TRY(launch_rbgs(L, 0, false, s));
+      WF_TRY(launch_rbgs(L, 1, true, s));
     }
     return WF_OK;
   }
@@ -2408,13 +2518,9 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
     WF_CKL("k_relax_smem");
     return WF_OK;
   }
-  const long half = (long)L.n * L.n * ((L.n + 1) / 2);
-  const int nb = mg_blocks(half);
   for (int sw = 0; sw < nsweeps; ++sw) {
-    WF_CK(launch_k(k_rbgs<T>, cells3(L.n, L.n, (L.n + 1) / 2), cell_block(), 0, s, L, 0));
-    WF_CKL("k_rbgs");
-    WF_CK(launch_k(k_rbgs<T>, cells3(L.n, L.n, (L.n + 1) / 2), cell_block(), 0, s, L, 1));
-    WF_CKL("k_rbgs");
+    WF_TRY(launch_rbgs(L, 0, sw > 0, s));
+    WF_TRY(launch_rbgs(L, 1, true, s));
   }
   return WF_OK;
 }
@@ -2423,7 +2529,7 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
 // to relax_split for both smoothings
 template <class T>
 static bool split_resident(const Lvl<T>& L, const wf_case& c) {
-  return L.tmp && (L.n & 1) == 0 && L.n > 24 && L.n >= split_min_n(sizeof(T) == 4) &&
+  return L.tmp && (L.n & 1) == 0 && L.n > 24 && L.n >= split_min_n() &&
          c.n_pre >= 1 && c.n_pre <= 12 && c.n_post >= 1 && c.n_post <= 12;
 }
 

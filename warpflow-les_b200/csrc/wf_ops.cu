@@ -595,8 +595,12 @@ static void shape_default(int kind, int n, int* a, int* b, int* c) {
   }
 }
 
+bool launch_shape_set(int kind, int n) {
+  return kind >= 0 && kind <= 1 && n >= 0 && n <= SHAPE_MAX_N && g_shape[kind][n][0];
+}
+
 void launch_shape(int kind, int n, int* a, int* b, int* c) {
-  const bool set = kind >= 0 && kind <= 1 && n >= 0 && n <= SHAPE_MAX_N && g_shape[kind][n][0];
+  const bool set = launch_shape_set(kind, n);
   shape_default(kind, n, a, b, c);
   if (set) {
     *a = g_shape[kind][n][0];

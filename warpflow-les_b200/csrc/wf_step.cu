@@ -25,16 +25,17 @@ namespace wf {
 
 static thread_local std::string g_err;
 thread_local long g_launches = 0;
-// Set while a stepper created with WF_STEP_SERIAL captures or launches.
+// Set while a stepper created with WF_STEP_SERIAL captures or launches: 1 no
+// programmatic dependent launch, 2 (WF_STEP_CHAIN) for the half-sweeps only.
 static thread_local int g_pdl_off = 0;
 
-bool pdl_enabled() {
+bool pdl_enabled(bool chain) {
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("WF_PDL");
     v = (e && e[0] == '0') ? 0 : 1;
   }
-  return v == 1 && !g_pdl_off;
+  return v == 1 && (!g_pdl_off || (chain && g_pdl_off == 2));
 }
 
 BatchCtx& batch_ctx() {
@@ -54,10 +55,13 @@ struct BatchScope {
   ~BatchScope() { batch_ctx() = prev; }
 };
 
-// Turns programmatic dependent launch off on this thread for one scope.
+// Turns programmatic dependent launch off on this thread for one scope
+// (chain: except for the half-sweeps).
 struct PdlOff {
   int prev;
-  explicit PdlOff(bool on) : prev(g_pdl_off) { if (on) g_pdl_off = 1; }
+  explicit PdlOff(bool on, bool chain = false) : prev(g_pdl_off) {
+    if (on) g_pdl_off = chain ? 2 : 1;
+  }
   ~PdlOff() { g_pdl_off = prev; }
 };
 
@@ -145,6 +149,7 @@ struct wf_stepper {
   wf_case c;
   int mode;     // 0 graph, 1 host loop
   int serial;   // WF_STEP_SERIAL: no programmatic dependent launch
+  int chain;    // WF_STEP_CHAIN: but for the half-sweeps
   int32_t counts[4];  // launches: prologue, calmas pass, multigrid part, epilogue
   cudaGraph_t graph;
   cudaGraphExec_t exec;
@@ -535,14 +540,16 @@ int wf_stepper_create(const wf_case* c, int32_t mode, wf_stepper** out) {
   if (!c || !out) return fail(WF_EINVAL, "null argument");
   *out = nullptr;
   WF_TRY(validate_case(*c));
-  if (mode & ~(1 | WF_STEP_SERIAL))
-    return fail(WF_EINVAL, "mode must be 0 (graph) or 1 (host loop), optionally | WF_STEP_SERIAL");
+  if (mode & ~(1 | WF_STEP_SERIAL | WF_STEP_CHAIN))
+    return fail(WF_EINVAL, "mode must be 0 (graph) or 1 (host loop), optionally | WF_STEP_SERIAL "
+                           "| WF_STEP_CHAIN");
   prepare_fills(c->n);   // the fill programs are built outside the capture
   wf_stepper* st = new wf_stepper();
   st->c = *c;
   st->mode = mode & 1;
   st->serial = (mode & WF_STEP_SERIAL) != 0;
-  PdlOff guard(st->serial);
+  st->chain = (mode & WF_STEP_CHAIN) != 0;
+  PdlOff guard(st->serial, st->chain);
   st->graph = nullptr;
   st->exec = nullptr;
   st->hflag = nullptr;
@@ -570,7 +577,7 @@ int wf_stepper_step(wf_stepper* st, void* stream) {
     return WF_OK;
   }
   const wf_case& c = st->c;
-  PdlOff guard(st->serial);
+  PdlOff guard(st->serial, st->chain);
   long l0 = g_launches;
   WF_TRY(step_prologue(c, s));
   st->counts[0] = (int32_t)(g_launches - l0);
@@ -597,11 +604,11 @@ int wf_stepper_step(wf_stepper* st, void* stream) {
 int wf_ensemble_create(const wf_case* cases, int32_t ncases, int32_t mode, wf_ensemble** out) {
   if (!cases || !out || ncases < 1) return fail(WF_EINVAL, "null argument or no cases");
   *out = nullptr;
-  if (mode & ~(WF_STEP_SERIAL | WF_ENS_BUCKETS))
+  if (mode & ~(WF_STEP_SERIAL | WF_ENS_BUCKETS | WF_STEP_CHAIN))
     return fail(WF_EINVAL, "ensemble mode: 0, WF_STEP_SERIAL and/or WF_ENS_BUCKETS");
   for (int i = 0; i < ncases; ++i) WF_TRY(validate_case(cases[i]));
   for (int i = 0; i < ncases; ++i) prepare_fills(cases[i].n);
-  PdlOff guard((mode & WF_STEP_SERIAL) != 0);
+  PdlOff guard((mode & WF_STEP_SERIAL) != 0, (mode & WF_STEP_CHAIN) != 0);
   wf_ensemble* en = new wf_ensemble();
   en->ncases = ncases;
   en->graph = nullptr;

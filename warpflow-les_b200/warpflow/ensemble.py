@@ -25,7 +25,7 @@ import torch
 from . import _abi
 from .config import case_from_dict
 from .fields import cuda_device
-from .solver import STEP_SERIAL, FlowSolver
+from .solver import STEP_CHAIN, STEP_SERIAL, FlowSolver
 
 ENS_BUCKETS = 4   # WF_ENS_BUCKETS
 from .topology import build_topology
@@ -100,7 +100,9 @@ class Ensemble:
         if single_graph and len(self.solvers) > 1:
             arr = (_abi.WfCase * len(self.solvers))(*[sv.case for sv in self.solvers])
             self._graph = ctypes.c_void_p()
-            mode = STEP_SERIAL | (ENS_BUCKETS if self.buckets else 0)
+            # a bucket's half-sweeps read the case table first, so they have
+            # nothing to do ahead of their wait
+            mode = STEP_SERIAL | (ENS_BUCKETS if self.buckets else STEP_CHAIN)
             _abi.call("wf_ensemble_create", arr, len(self.solvers), mode,
                       ctypes.byref(self._graph))
         ns = max(1, min(nstreams, len(self.solvers)))

@@ -37,19 +37,19 @@ ALFARK = (0.5, 1.0)  # Heun RK2 stage coefficients (reference solver.py:26)
 
 STEP_MODES = {"graph": 0, "host": 1}
 STEP_SERIAL = 2   # WF_STEP_SERIAL: no programmatic dependent launch
+STEP_CHAIN = 8    # WF_STEP_CHAIN: but for the half-sweeps
 
 
 class FlowSolver:
     def __init__(self, cfg, topo, device, step_mode=None, serial=True):
         """`serial` (the default) builds the step without programmatic
-        dependent launch: each kernel's CTAs become resident only after the
-        previous kernel finished.  Measured on B200 the single-case step
-        graph is about 1.3 % faster that way at 80^3 (1.008 against 1.024 ms
-        and 1.019 against 1.031 ms in two runs; 256^3 and 512^3 unchanged),
-        and many solvers stepping concurrently need it (waiting CTAs would
-        hold SMs other streams could use).  `serial=False` launches the
-        step's kernels with programmatic dependent launch; the results are
-        the same bits."""
+        dependent launch, but for the multigrid half-sweeps: every other
+        kernel's CTAs become resident only after the previous kernel
+        finished, and solvers stepping concurrently find the SMs free.
+        Measured on B200, us per step, none / half-sweeps / all kernels:
+        80^3 872 / 812 / 814 when the half-sweeps began to read their
+        right-hand side ahead of the wait.  `serial=False` launches all of
+        the step's kernels with it; the results are the same bits."""
         self.cfg = cfg
         self.topo = topo
         dev = cuda_device(device)
@@ -105,7 +105,7 @@ class FlowSolver:
         self.step_mode = mode
         self._stepper = ctypes.c_void_p()
         _abi.call("wf_stepper_create", ctypes.byref(self.case),
-                  STEP_MODES[mode] | (STEP_SERIAL if serial else 0),
+                  STEP_MODES[mode] | (STEP_SERIAL | STEP_CHAIN if serial else 0),
                   ctypes.byref(self._stepper))
 
     def _init_state(self):
