@@ -454,13 +454,14 @@ __global__ void __launch_bounds__(1024) k_relax_smem(Lvl<T> L0, int nsweeps, con
 // independent), phase 2 updates the column top-down and publishes the new
 // values, so no shared-memory store sits between two loads.  The sum keeps
 // the reference's term order aw W + ae E + as S + an N + ab B + at T.
-template <class T, int NC, int KP, bool RHS_SMEM>
+template <class T, int NC, int KP, bool RHS_SMEM, bool EXACT = false>
 __device__ __forceinline__ void half_sweep_cols(const T* __restrict__ oth, T* __restrict__ own,
                                                 int PLANE, int me, int oW, int oE, int oS,
                                                 int oN, T aw, T ae, T as, T an, T az, T inv_in,
                                                 T inv_lo, T inv_hi, T (&ph)[NC],
                                                 const T (&rh)[RHS_SMEM ? 1 : NC],
-                                                const T* __restrict__ srh) {
+                                                const T* __restrict__ srh, T ap_in = T(0),
+                                                T ap_edge = T(0)) {
   constexpr int NK = (NC - KP + 1) / 2;
   T nb[NK];
 #pragma unroll
@@ -480,7 +481,9 @@ __device__ __forceinline__ void half_sweep_cols(const T* __restrict__ oth, T* __
     if (k > 0) sum = sum + az * ph[k - 1];
     if (k < NC - 1) sum = sum + az * ph[k + 1];
     const T r = RHS_SMEM ? rr[RHS_SMEM ? t : 0] : rh[RHS_SMEM ? 0 : k];
-    const T x = (r - sum) * (k == 0 ? inv_lo : (k == NC - 1 ? inv_hi : inv_in));
+    const T inv = k == 0 ? inv_lo : (k == NC - 1 ? inv_hi : inv_in);
+    const T x = EXACT ? div_by_recip(r - sum, k == 0 || k == NC - 1 ? ap_edge : ap_in, inv)
+                      : (r - sum) * inv;
     ph[k] = x;
   }
 #pragma unroll
@@ -779,7 +782,8 @@ static int launch_coarse_cluster(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
 // nobody waits for a memory fence or for CTAs it does not exchange with.
 // Ordering: a neighbour can only produce the next values of a colour after
 // receiving the values this CTA computes from the current ones, so a halo
-// cell is never overwritten while it may still be read.
+// cell is never overwritten while it may still be read.  EXACT: the quotient
+// of k_rbgs instead of the product with the reciprocal.
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return (uint32_t)__cvta_generic_to_shared(p);
 }
@@ -841,7 +845,7 @@ __device__ __forceinline__ void st_async(uint32_t raddr, float v, uint32_t rmbar
 // much less when spinning)
 constexpr int MBAR_WAIT_TRIES = 1 << 22;
 
-template <class T, int NC, int NCL>
+template <class T, int NC, int NCL, bool EXACT>
 __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     k_coarse_p2p(Lvl<T> L, int nsweeps, int wmode) {
   pdl_entry();
@@ -882,6 +886,7 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
   const T inv_in = T(1) / (-(aw + ae + as + an + az + az));
   const T inv_lo = T(1) / (-(aw + ae + as + an + T(0) + az));
   const T inv_hi = T(1) / (-(aw + ae + as + an + az + T(0)));
+  const T ap_in = -(aw + ae + as + an + az + az), ap_edge = -(aw + ae + as + an + az);
   const bool sendW = active && il == 0 && rank > 0;
   const bool sendE = active && il == NCL - 1 && rank < C - 1;
   // this column's halo slot in the neighbour (same parity array, k = 0)
@@ -939,11 +944,13 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     const int kp = (1 + g + (t & 1)) & 1;
     if (active) {
       if (kp == 0)
-        half_sweep_cols<T, NC, 0, false>(oth, own, PL, me, oW, oE, oS, oN, aw, ae, as, an, az,
-                                         inv_in, inv_lo, inv_hi, ph, rh, nullptr);
+        half_sweep_cols<T, NC, 0, false, EXACT>(oth, own, PL, me, oW, oE, oS, oN, aw, ae, as, an,
+                                                az, inv_in, inv_lo, inv_hi, ph, rh, nullptr,
+                                                ap_in, ap_edge);
       else
-        half_sweep_cols<T, NC, 1, false>(oth, own, PL, me, oW, oE, oS, oN, aw, ae, as, an, az,
-                                         inv_in, inv_lo, inv_hi, ph, rh, nullptr);
+        half_sweep_cols<T, NC, 1, false, EXACT>(oth, own, PL, me, oW, oE, oS, oN, aw, ae, as, an,
+                                                az, inv_in, inv_lo, inv_hi, ph, rh, nullptr,
+                                                ap_in, ap_edge);
       const uint32_t mc = (uint32_t)(t & 1);
       if (sendW) {
 #pragma unroll
@@ -977,12 +984,12 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
   }
 }
 
-template <class T, int NC, int NCL>
+template <class T, int NC, int NCL, bool EXACT = false>
 static int launch_coarse_p2p(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
   if (batch_ctx().tab) return fail(WF_EUNSUPPORTED, "cluster and cooperative relaxes do not run in a bucket");
   using S = ClusterShape<NC, NCL>;
   const size_t sb = 2ull * NC * S::PL * sizeof(T);
-  auto kern = k_coarse_p2p<T, NC, NCL>;
+  auto kern = k_coarse_p2p<T, NC, NCL, EXACT>;
   WF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb));
   if (S::C > 8) WF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
   cudaLaunchConfig_t cfg = {};
@@ -1019,6 +1026,26 @@ static int try_coarse_p2p_thin(const Lvl<T>& L, int nsweeps, cudaStream_t s, int
     case 24: *rc = launch_coarse_p2p<T, 24, 2>(L, nsweeps, s); return 1;
     case 28: *rc = launch_coarse_p2p<T, 28, 2>(L, nsweeps, s); return 1;
     case 32: *rc = launch_coarse_p2p<T, 32, 2>(L, nsweeps, s); return 1;
+    default: return 0;
+  }
+}
+
+// Even edges that have neither an operator nor a strategy of their own: many
+// sweeps run in a cluster with the exact quotient, so that the bits are those of
+// k_relax_smem (one CTA, runtime index divisions) and k_rbgs (two launches a
+// sweep), which ran them before.  us per 300 sweeps, FP64, before / now: 10^3
+// 427 / 279, 14^3 1003 / 345, 18^3 1787 / 393, 22^3 3137 / 406, 26^3 1307 /
+// 469, 30^3 1312 / 584 (FP32 26^3 and 30^3 took 3-5 ms in one CTA); 6^3 stays in
+// one CTA (237 / 259).  The slabs are those that measured fastest.
+template <class T>
+static int try_coarse_exact(const Lvl<T>& L, int nsweeps, cudaStream_t s, int* rc) {
+  switch (L.n) {
+    case 10: *rc = launch_coarse_p2p<T, 10, 1, true>(L, nsweeps, s); return 1;
+    case 14: *rc = launch_coarse_p2p<T, 14, 2, true>(L, nsweeps, s); return 1;
+    case 18: *rc = launch_coarse_p2p<T, 18, 3, true>(L, nsweeps, s); return 1;
+    case 22: *rc = launch_coarse_p2p<T, 22, 2, true>(L, nsweeps, s); return 1;
+    case 26: *rc = launch_coarse_p2p<T, 26, 2, true>(L, nsweeps, s); return 1;
+    case 30: *rc = launch_coarse_p2p<T, 30, 3, true>(L, nsweeps, s); return 1;
     default: return 0;
   }
 }
@@ -2481,6 +2508,7 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
     if (nsweeps > 12 && strat == 2 && try_coarse_p2p<T>(L, nsweeps, s, &rc)) return rc;
     if (nsweeps > 12 && strat == 1 && try_coarse_cluster<T>(L, nsweeps, s, &rc)) return rc;
     if (try_coarse<T>(L, nsweeps, s, &rc)) return rc;
+    if (!bucket && nsweeps > 12 && try_coarse_exact<T>(L, nsweeps, s, &rc)) return rc;
   }
   if (L.tmp && (L.n & 1) == 0 && L.n >= split_min_n())
     return relax_split<T>(L, nsweeps, rhs_ready, s);
