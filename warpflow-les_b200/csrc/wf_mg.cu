@@ -1067,6 +1067,297 @@ static int try_coarse_p2p(const Lvl<T>& L, int nsweeps, cudaStream_t s, int* rc)
   }
 }
 
+// ---- the coarsest relax from zero as a polynomial ---------------------------
+// From phi = 0 the first sweep gives x_A = b_A / ap, x_B1 = v_B / ap, and every
+// later sweep maps x_B <- x_B1 + G x_B with G = D_B^-1 A_BA D_A^-1 A_AB (see
+// below, the coarse operator).  After m further sweeps x_B = p(G) x_B1,
+// p(z) = sum_{s<=m} z^s, and the spectrum of G lies in [0, 1].  In Chebyshev
+// polynomials of 2z - 1, z^s = 4^-s (C(2s, s) + 2 sum_k C(2s, s-k) T_k): the
+// coefficients of p are positive and fall off like exp(-k^2 / m), so p is a sum
+// of about 5.8 sqrt(m) terms to the last bit of an FP64 result (degree 97 in
+// place of 283 sweeps), summed by Clenshaw's recurrence (C. W. Clenshaw, "A note
+// on the summation of Chebyshev series", MTAC 9, 1955).  A term costs one sweep
+// with a zero rhs.  The last CHEB_TAIL + 1 sweeps run as such: they damp the
+// recurrence's rounding errors, and the result stays as close to exact
+// arithmetic as the sweeps' (about 1e-15 of its size).
+// us per 300-sweep relax, FP64, sweeps / polynomial: 10^3 279 / 140, 18^3 393 /
+// 183, 24^3 380 / 206, 32^3 466 / 270.
+constexpr int CHEB_MAX = 128;
+constexpr int CHEB_TAIL = 16;
+struct ChebCoef {
+  double c[CHEB_MAX];
+  int deg;
+};
+
+// coefficients of sum_{s<m} ((1 + t) / 2)^s, cut where the rest is below an ulp
+// of the sum (m); deg < 0 when CHEB_MAX terms do not reach that.  The row of
+// 4^-s C(2s, s-k) is a random walk's distribution: positive terms only.
+static const ChebCoef& cheb_coef(int m) {
+  static thread_local ChebCoef last{{}, -2};
+  static thread_local int last_m = -1;
+  if (last_m == m) return last;
+  std::vector<double> p(CHEB_MAX + 2, 0.0), q(CHEB_MAX + 2, 0.0), sum(CHEB_MAX + 2, 0.0);
+  p[0] = 1.0;
+  for (int s = 0; s < m; ++s) {
+    for (int k = 0; k <= CHEB_MAX; ++k) sum[k] += p[k];
+    for (int k = 0; k <= CHEB_MAX; ++k)
+      q[k] = 0.5 * p[k] + 0.25 * ((k ? p[k - 1] : p[1]) + p[k + 1]);
+    std::swap(p, q);
+  }
+  last.deg = -1;
+  double rest = 0.0;
+  for (int k = CHEB_MAX; k >= 1; --k) {
+    rest += 2.0 * sum[k];
+    if (rest > 1e-17 * m) {
+      if (k < CHEB_MAX) last.deg = k;
+      break;
+    }
+  }
+  for (int k = 0; k < CHEB_MAX; ++k) last.c[k] = (k ? 2.0 : 1.0) * sum[k];
+  last_m = m;
+  return last;
+}
+
+// one colour of one column, as half_sweep_cols: MODE 0 with the rhs, MODE 1 with
+// a zero rhs, MODE 2 with a zero rhs followed by the recurrence (ph the term
+// before, bp the one before that, x1 the first sweep's cells; the last one
+// closes the sum)
+template <int NC, int KP, int MODE>
+__device__ __forceinline__ void cheb_cols(const double* __restrict__ oth, double* __restrict__ own,
+                                          int PLANE, int me, int oW, int oE, int oS, int oN,
+                                          double aw, double ae, double as, double an, double az,
+                                          double inv_in, double inv_edge, double ap_in,
+                                          double ap_edge, double (&ph)[NC], const double (&rh)[NC],
+                                          double (&bp)[NC / 2], const double (&x1)[NC / 2],
+                                          double ck, bool last) {
+  constexpr int NK = (NC - KP + 1) / 2;
+  double nb[NK];
+#pragma unroll
+  for (int t = 0; t < NK; ++t) {
+    const double* pl = oth + (KP + 2 * t) * PLANE;
+    nb[t] = aw * pl[oW] + ae * pl[oE] + as * pl[oS] + an * pl[oN];
+  }
+#pragma unroll
+  for (int t = 0; t < NK; ++t) {
+    const int k = KP + 2 * t;
+    double sum = nb[t];
+    if (k > 0) sum = sum + az * ph[k - 1];
+    if (k < NC - 1) sum = sum + az * ph[k + 1];
+    const bool edge = k == 0 || k == NC - 1;
+    double x = div_by_recip(MODE == 0 ? rh[k] - sum : -sum, edge ? ap_edge : ap_in,
+                            edge ? inv_edge : inv_in);
+    if (MODE == 2) {
+      x = fma(ck, x1[t], (last ? 2.0 * x - ph[k] : 4.0 * x - 2.0 * ph[k]) - bp[t]);
+      bp[t] = ph[k];
+    }
+    ph[k] = x;
+  }
+#pragma unroll
+  for (int t = 0; t < NK; ++t) own[(KP + 2 * t) * PLANE + me] = ph[KP + 2 * t];
+}
+
+// the relax above on the slabs of k_coarse_p2p
+template <int NC, int NCL>
+__global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
+    k_coarse_cheb(Lvl<double> L0, const __grid_constant__ ChebCoef C, int wmode, const Batch bt) {
+  pdl_entry();
+  if (bt_skip(bt)) return;   // the case's whole cluster
+  const Lvl<double> L = rebase(L0, bt);
+  using T = double;
+  using S = ClusterShape<NC, NCL>;
+  constexpr int H = S::H, HALF = S::HALF, GROUP = S::GROUP, PL = S::PL, NB = S::C;
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank();
+  extern __shared__ __align__(16) unsigned char smraw[];
+  __shared__ __align__(8) unsigned long long mbar[2];
+  __shared__ int s_bail;
+  T* sp = reinterpret_cast<T*>(smraw);
+  const int tid = threadIdx.x;
+  const uint32_t mb[2] = {smem_u32(&mbar[0]), smem_u32(&mbar[1])};
+  const int nbr = (rank > 0 ? 1 : 0) + (rank < NB - 1 ? 1 : 0);
+  const uint32_t tx = (uint32_t)(nbr * (NC * NC / 2) * sizeof(T));
+  if (tid == 0) {
+    mbar_init(mb[0], 1);
+    mbar_init(mb[1], 1);
+    s_bail = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  for (int t = tid; t < 2 * NC * PL; t += blockDim.x) sp[t] = T(0);
+  const int g = tid / GROUP;
+  const int q = tid - g * GROUP;
+  const bool active = q < HALF;
+  const int il = active ? q / H : 0;
+  const int m = active ? q - il * H : 0;
+  const int i = rank * NCL + il;
+  const int j = 2 * m + ((i + g) & 1);
+  T* own = sp + g * NC * PL;
+  const T* oth = sp + (1 - g) * NC * PL;
+  const int me = (il + 1) * H + m;
+  const int oW = me - H, oE = me + H;
+  const int oS = j > 0 ? (il + 1) * H + ((j - 1) >> 1) : me;
+  const int oN = j < NC - 1 ? (il + 1) * H + ((j + 1) >> 1) : me;
+  const T aw = i > 0 ? L.ax : T(0), ae = i < NC - 1 ? L.ax : T(0);
+  const T as = j > 0 ? L.ay : T(0), an = j < NC - 1 ? L.ay : T(0);
+  const T az = L.az;
+  const T ap_in = -(aw + ae + as + an + az + az), ap_edge = -(aw + ae + as + an + az);
+  const T inv_in = T(1) / ap_in, inv_edge = T(1) / ap_edge;
+  const bool sendW = active && il == 0 && rank > 0;
+  const bool sendE = active && il == NCL - 1 && rank < NB - 1;
+  const uint32_t own_u32 = smem_u32(own);
+  uint32_t aW = 0, aE = 0, mW[2] = {0, 0}, mE[2] = {0, 0};
+  if (sendW) {
+    aW = mapa_u32(own_u32 + (uint32_t)(((NCL + 1) * H + m) * sizeof(T)), rank - 1);
+    mW[0] = mapa_u32(mb[0], rank - 1);
+    mW[1] = mapa_u32(mb[1], rank - 1);
+  }
+  if (sendE) {
+    aE = mapa_u32(own_u32 + (uint32_t)(m * sizeof(T)), rank + 1);
+    mE[0] = mapa_u32(mb[0], rank + 1);
+    mE[1] = mapa_u32(mb[1], rank + 1);
+  }
+  T ph[NC], rh[NC], bp[NC / 2], x1[NC / 2];
+  const long c0 = lid(L, i + 1, j + 1, 1);
+#pragma unroll
+  for (int k = 0; k < NC; ++k) {
+    ph[k] = T(0);
+    rh[k] = active ? L.rhs[c0 + k] : T(0);
+  }
+#pragma unroll
+  for (int k = 0; k < NC / 2; ++k) bp[k] = x1[k] = T(0);
+  if (tid == 0) {
+    mbar_arrive_expect_tx(mb[0], tx);
+    mbar_arrive_expect_tx(mb[1], tx);
+  }
+  cl.sync();  // barriers armed and planes zeroed in every CTA
+  // the first sweep, deg terms, CHEB_TAIL + 1 sweeps
+  const int nh = 2 * (1 + C.deg + CHEB_TAIL + 1);
+  bool bailed = false;
+  for (int t = 0; t < nh; ++t) {
+    if (t > 0) {
+      const int c = (t - 1) & 1;
+      const uint32_t par = (uint32_t)(((t - 1) >> 1) & 1);
+      bool ok = false;
+      for (int it = 0; it < MBAR_WAIT_TRIES && !ok; ++it) ok = mbar_try_wait(mb[c], par, wmode);
+      if (!ok) s_bail = 1;
+      if (tid == 0 && t + 1 < nh) mbar_arrive_expect_tx(mb[c], tx);
+    }
+    __syncthreads();
+    if (s_bail) {
+      bailed = true;
+      break;
+    }
+    const int kp = (1 + g + (t & 1)) & 1;
+    const int term = t >> 1;                       // 0: the first sweep, 1 .. deg: the sum
+    const bool plain = term == 0 || term > C.deg;
+    if (active) {
+      const double ck = C.c[max(C.deg - term, 0)];
+#define WF_CHEB(KP, MODE)                                                                     \
+  cheb_cols<NC, KP, MODE>(oth, own, PL, me, oW, oE, oS, oN, aw, ae, as, an, az, inv_in, inv_edge, \
+                          ap_in, ap_edge, ph, rh, bp, x1, ck, term == C.deg)
+      if (plain) {
+        if (kp == 0) WF_CHEB(0, 0); else WF_CHEB(1, 0);
+        if (t == 1) {   // the B cells of the first sweep; the sum starts with the highest term
+#pragma unroll
+          for (int k = 0; k < NC; ++k)
+            if ((k & 1) == kp) {
+              x1[k >> 1] = ph[k];
+              ph[k] = ck * ph[k];
+              own[k * PL + me] = ph[k];
+            }
+        }
+      } else if (!(t & 1)) {
+        if (kp == 0) WF_CHEB(0, 1); else WF_CHEB(1, 1);
+      } else {
+        if (kp == 0) WF_CHEB(0, 2); else WF_CHEB(1, 2);
+      }
+#undef WF_CHEB
+      const uint32_t mc = (uint32_t)(t & 1);
+      if (sendW) {
+#pragma unroll
+        for (int k = 0; k < NC; ++k)
+          if ((k & 1) == kp) st_async(aW + (uint32_t)(k * PL * sizeof(T)), ph[k], mW[mc]);
+      }
+      if (sendE) {
+#pragma unroll
+        for (int k = 0; k < NC; ++k)
+          if ((k & 1) == kp) st_async(aE + (uint32_t)(k * PL * sizeof(T)), ph[k], mE[mc]);
+      }
+    }
+  }
+  if (!bailed) {
+    // the neighbours' last pushes must land before exit
+    const int c = (nh - 1) & 1;
+    const uint32_t par = (uint32_t)(((nh - 1) >> 1) & 1);
+    bool ok = false;
+    for (int it = 0; it < MBAR_WAIT_TRIES && !ok; ++it) ok = mbar_try_wait(mb[c], par, wmode);
+    if (!ok) s_bail = 1;
+  }
+  __syncthreads();
+  if (s_bail && tid == 0 && L.err) atomicExch(L.err, (int)WF_ST_WAIT_TIMEOUT);
+  cl.sync();
+  if (!active) return;
+#pragma unroll
+  for (int k = 0; k < NC; ++k) {
+    const long c = c0 + k;
+    L.phi[c] = ph[k];
+    ring_mirror(L, i, j, k, c, ph[k]);
+  }
+}
+
+template <int NC, int NCL>
+static int launch_coarse_cheb(const Lvl<double>& L, const ChebCoef& C, cudaStream_t s) {
+  using S = ClusterShape<NC, NCL>;
+  const size_t sb = 2ull * NC * S::PL * sizeof(double);
+  auto kern = k_coarse_cheb<NC, NCL>;
+  const BatchCtx& bc = batch_ctx();   // a cluster per case
+  const Batch b{bc.tab, 1, bc.skip};
+  WF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb));
+  if (S::C > 8) WF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(S::C, 1, bc.tab ? bc.ncases : 1);
+  cfg.blockDim = dim3(S::THREADS, 1, 1);
+  cfg.dynamicSmemBytes = sb;
+  cfg.stream = s;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = S::C;
+  at[0].val.clusterDim.y = 1;
+  at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl_enabled() ? 2 : 1;
+  WF_CK(cudaLaunchKernelEx(&cfg, kern, L, C, 1, b));
+  WF_CKL("k_coarse_cheb");
+  return WF_OK;
+}
+
+// the coarsest relax of an FP64 level whose phi is zero, where the polynomial
+// serves it, in a bucket too (a case computes the same bits alone and in one):
+// where it saves at least a third of the sweeps
+static int try_coarse_cheb(const Lvl<double>& L, int nsweeps, cudaStream_t s, int* rc) {
+  if (nsweeps < 64) return 0;
+  const ChebCoef& C = cheb_coef(nsweeps - 1 - CHEB_TAIL);
+  if (C.deg < 1 || 3 * (C.deg + 2 + CHEB_TAIL) > 2 * nsweeps) return 0;
+  switch (L.n) {
+    case 10: *rc = launch_coarse_cheb<10, 1>(L, C, s); return 1;
+    case 12: *rc = launch_coarse_cheb<12, 2>(L, C, s); return 1;
+    case 14: *rc = launch_coarse_cheb<14, 2>(L, C, s); return 1;
+    case 16: *rc = launch_coarse_cheb<16, 2>(L, C, s); return 1;
+    case 18: *rc = launch_coarse_cheb<18, 3>(L, C, s); return 1;
+    case 20: *rc = launch_coarse_cheb<20, 4>(L, C, s); return 1;
+    case 22: *rc = launch_coarse_cheb<22, 2>(L, C, s); return 1;
+    case 24: *rc = launch_coarse_cheb<24, 2>(L, C, s); return 1;
+    case 26: *rc = launch_coarse_cheb<26, 2>(L, C, s); return 1;
+    case 28: *rc = launch_coarse_cheb<28, 2>(L, C, s); return 1;
+    case 30: *rc = launch_coarse_cheb<30, 3>(L, C, s); return 1;
+    case 32: *rc = launch_coarse_cheb<32, 2>(L, C, s); return 1;
+    default: return 0;
+  }
+}
+static int try_coarse_cheb(const Lvl<float>&, int, cudaStream_t, int*) { return 0; }
+
 // mid-size levels (a few sweeps of 28^3..48^3): the whole level resident in
 // the distributed shared memory of one cluster, so a 6-sweep relax is one
 // launch instead of twelve.  Off by default (WF_MID=1 turns it on): inside
@@ -2491,9 +2782,15 @@ constexpr size_t SMEM_CAP = 220 * 1024;
 
 // rhs_ready: the level's rhs is unchanged since its last relax, so a split
 // copy of it made then can be reused
+// zero: the level's phi is zero (a coarsest level after the restriction)
 template <class T>
-static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = false) {
+static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = false,
+                 bool zero = false) {
   if (nsweeps <= 0) return WF_OK;
+  {
+    int rc = WF_OK;
+    if (zero && try_coarse_cheb(L, nsweeps, s, &rc)) return rc;
+  }
   // a bucket launch serves many cases through their table: only kernels that
   // take one (the one-CTA column kernel, split and plain sweeps, the
   // shared-memory relax) run there
@@ -2592,7 +2889,8 @@ static int vcycle(std::vector<Lvl<T>>& lv, const wf_case& c, cudaStream_t s,
     else if (res[l])
       WF_TRY(split_sweeps(lv[l], c.n_pre, s));
     else
-      WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, l == 0 && rhs0_ready));
+      WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, l == 0 && rhs0_ready,
+                   l > 0 && l == L - 1));
   }
   for (int l = L - 2; l >= 0; --l) {
     // fine levels from 64: one thread per coarse cell (fewer loads); smaller
@@ -2928,7 +3226,7 @@ int mg_coarse_solve_pair(const wf_case& c, double* phi, const double* rhs, cudaS
   WF_CKL("k_zero");
   if (c.mg_cop && c.mg_cop_part && !c.mg_fp32 && c.n_coarse >= 2 && cop_size_ok(L.n))
     return apply_coarse_op<double>(L, (const double*)c.mg_cop, (double*)c.mg_cop_part, s);
-  return relax<double>(L, c.n_coarse, s);
+  return relax<double>(L, c.n_coarse, s, false, true);
 }
 
 __global__ void k_refill(Lvl<double> L) {
@@ -3083,7 +3381,7 @@ static int vcycle_fixed(Lvl<double>* lv, int L, const wf_case& c, cudaStream_t s
           lv[l - 1], const_cast<double*>(lv[l].rhs), lv[l]));
       WF_CKL("k_restrict");
     }
-    WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s));
+    WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, false, l > 0 && l == L - 1));
   }
   for (int l = L - 2; l >= 0; --l) {
     WF_CK(launch_k(k_prolong<double>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s, 
