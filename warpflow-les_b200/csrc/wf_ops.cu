@@ -57,12 +57,16 @@ static inline Geo geo_of(int n) {
 }
 
 // reductions over the n^3 real cells: 1-D CTAs of 32 (k) x 8 (j) threads,
-// grid (k runs, j groups, G) with each CTA stepping through planes i by G;
-// G keeps the grid near 32 CTAs per SM: enough independent planes in flight,
-// few enough CTAs meeting at the reduction atomics
+// grid (k runs, j groups, G) with each CTA stepping through planes i by G: few
+// CTAs, because every one meets the others at the reduction words and the
+// ticket, but enough planes in flight.  us of k_checkdt / k_calmas at 32, 16, 8
+// and 4 CTAs per SM: 80^3 14.9 / 11.6, 14.4 / 11.0, 10.6 / 9.2, 11.4 / 11.2;
+// 128^3 29.0 / 22.7, 21.7 / 18.1, 20.7 / 16.1, 22.7 / 23.7; 256^3 132 / 135,
+// 126 / 130, 169 / 129, 165 / 219 (before the maxima read the word first: 80^3
+// 19.3 / 11.0, 256^3 141 / 135)
 static inline dim3 reduce_grid(int n) {
   const int gx = (n + 31) / 32, gy = (n + 7) / 8;
-  const int g = std::max(1, std::min(n, (148 * 32) / (gx * gy)));
+  const int g = std::max(1, std::min(n, 148 * (n >= 192 ? 16 : 8) / (gx * gy)));
   return dim3(gx, gy, g);
 }
 
@@ -145,6 +149,31 @@ int launch_init_noise(double* u, double* v, double* w, int n, double amp, int se
   return WF_OK;
 }
 
+// the CTA's maxima of N order keys into global words.  A CTA whose maximum does
+// not exceed the word it reads leaves the word alone: the words only grow while
+// the launch runs, and same-address atomics are served one by one
+template <int N>
+__device__ __forceinline__ void reduce_keys(unsigned long long (&key)[N],
+                                            unsigned long long* word) {
+  __shared__ unsigned long long part[N][TPB / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < N; ++q) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) key[q] = max(key[q], __shfl_xor_sync(0xffffffffu, key[q], o));
+    if (lane == 0) part[q][warp] = key[q];
+  }
+  __syncthreads();
+  if (threadIdx.x < N) {
+    unsigned long long m = part[threadIdx.x][0];
+#pragma unroll
+    for (int w = 1; w < TPB / 32; ++w) m = max(m, part[threadIdx.x][w]);
+    volatile unsigned long long* vw = word + threadIdx.x;
+    if (m > *vw) atomicMax(word + threadIdx.x, m);
+    __threadfence();   // before the CTA's ticket
+  }
+}
+
 // --------------------------------------------------------------------------
 // checkdt (solver.py:122-150, kernels.py:374-402): max|u|, max|v|, max|w|
 // and the viscous/advective min in one pass; the last block finishes the
@@ -153,7 +182,6 @@ int launch_init_noise(double* u, double* v, double* w, int n, double amp, int se
 __global__ void __launch_bounds__(TPB) k_checkdt(const wf_case c, Geo g, const Divs dv,
                                                 const Batch bt) {
   pdl_entry();
-  __shared__ double sm[32];
   const double* u = bt_fld(c, bt, WF_U);
   const double* v = bt_fld(c, bt, WF_V);
   const double* w = bt_fld(c, bt, WF_W);
@@ -170,7 +198,6 @@ __global__ void __launch_bounds__(TPB) k_checkdt(const wf_case c, Geo g, const D
   // of one per cell, the same bits for every input.
   double mu = 0.0, mv = 0.0, mw = 0.0;
   unsigned long long kx = 0ull;
-  __shared__ unsigned long long skx[32];
   const int k = NPL + blockIdx.x * 32 + (threadIdx.x & 31);
   const int j = NPL + blockIdx.y * 8 + (threadIdx.x >> 5);
   const bool in = k < NPL + g.n && j < NPL + g.n;
@@ -189,22 +216,9 @@ __global__ void __launch_bounds__(TPB) k_checkdt(const wf_case c, Geo g, const D
                      1.0e-30;
     if (x == x) kx = max(kx, okey(x) ^ 0x8000000000000000ull);
   }
-  mu = block_max(mu, sm);
-  mv = block_max(mv, sm);
-  mw = block_max(mw, sm);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) kx = max(kx, __shfl_xor_sync(0xffffffffu, kx, o));
-  if ((threadIdx.x & 31) == 0) skx[threadIdx.x >> 5] = kx;
-  __syncthreads();
-  if (threadIdx.x == 0)
-    for (int q = 1; q < (int)((blockDim.x + 31) >> 5); ++q) kx = max(kx, skx[q]);
   wf_scalars* sc = bt_sc(c, bt);
-  if (threadIdx.x == 0) {
-    atomicMax(&sc->red[0], okey(mu));
-    atomicMax(&sc->red[1], okey(mv));
-    atomicMax(&sc->red[2], okey(mw));
-    atomicMax(&sc->red[3], kx);
-  }
+  unsigned long long key[4] = {okey(mu), okey(mv), okey(mw), kx};
+  reduce_keys<4>(key, sc->red);
   if (!last_block(&sc->ticket, gridDim.x * gridDim.y * bt_gz(bt))) return;
   if (threadIdx.x != 0) return;
   const double umax = okey_inv(atomicAdd(&sc->red[0], 0ull));
@@ -757,7 +771,6 @@ __global__ void __launch_bounds__(TPB) k_calmas(const wf_case c, Geo g,
                                                unsigned long long h_loop, const Divs dv,
                                                const Batch bt) {
   pdl_entry();
-  __shared__ double sm[32];
   const double* u = bt_fld(c, bt, WF_U);
   const double* v = bt_fld(c, bt, WF_V);
   const double* w = bt_fld(c, bt, WF_W);
@@ -788,8 +801,8 @@ __global__ void __launch_bounds__(TPB) k_calmas(const wf_case c, Geo g,
     su[id] = div_by_recip(fact, dt, rdt);
     mloc = fmax(mloc, fabs(fact * dx * dy * dz));
   }
-  mloc = block_max(mloc, sm);
-  if (threadIdx.x == 0) atomicMax(&sc->red[4], okey(mloc));
+  unsigned long long key[1] = {okey(mloc)};
+  reduce_keys<1>(key, sc->red + 4);
   if (!last_block(&sc->ticket, gridDim.x * gridDim.y * bt_gz(bt))) return;
   if (threadIdx.x != 0) return;
   const double rmax = okey_inv(atomicAdd(&sc->red[4], 0ull));
