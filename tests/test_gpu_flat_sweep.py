@@ -1,7 +1,8 @@
-"""The half-sweeps on the row-parity-split copy with the cells numbered flat
-(levels from 64 to below 104 cells, one or two cells per thread) give the bits
-of the in-place half-sweeps, in both precisions and at the edges of each
-range; the in-place ones follow the oracle's sweeps."""
+"""The half-sweeps on the row-parity-split copy -- with the cells numbered flat
+(levels from 64 to below 104 cells, one or two cells per thread), by rows, and
+in pairs marching through planes (multiples of 4 from 144) -- give the bits of
+the in-place half-sweeps, in both precisions and at the edges of each range;
+the in-place ones follow the oracle's sweeps."""
 import ctypes
 
 import numpy as np
@@ -19,7 +20,8 @@ def _mg(n, levels, precision):
     return Multigrid(cfg, build_topology(cfg), "cuda:0", 1.0 / n, 1.0 / n, 1.0 / n)
 
 
-@pytest.mark.parametrize("n", [62, 64, 66, 84, 86, 102, 104, 106])
+@pytest.mark.parametrize("n", [62, 64, 66, 84, 86, 102, 104, 106, 140, 144, 146, 172, 176,
+                               180, 260])
 def test_relax_on_split_copy_equals_in_place(n):
     mg = _mg(n, 1, "fp64")
     rng = np.random.default_rng(n)
@@ -56,7 +58,8 @@ def test_relax_in_place_follows_the_oracle(n):
     assert np.abs(got - lev.phi)[1:-1, 1:-1, 1:-1].max() <= 1e-14 * np.abs(lev.phi).max()
 
 
-@pytest.mark.parametrize("n,levels", [(64, 3), (80, 3), (96, 3), (128, 4)])
+@pytest.mark.parametrize("n,levels", [(64, 3), (80, 3), (96, 3), (128, 4), (144, 4), (184, 4),
+                                      (256, 5)])
 def test_mixed_solve_on_split_copies_equals_in_place(n, levels):
     from warpflow import _abi
     from warpflow.fields import DeviceField

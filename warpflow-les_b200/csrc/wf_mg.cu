@@ -54,6 +54,20 @@ struct Lvl {
 };
 constexpr int LV_PP = 16, LV_SPLIT = 32;
 
+// The row-parity-split copies of a level in its scratch of 2 (n+2)^3 elements.
+// Both start at an odd element, because a colour's real cells of a row start at
+// an odd element of the copy (for n a multiple of 4): they are then aligned for
+// loads of two.  The last element of the copy of phi shares its place with the
+// first ones of the copy of rhs; all of these are edges of the ring, which
+// nothing reads from a level that has an rhs ring.
+template <class T>
+__host__ __device__ __forceinline__ T* split_phi(T* tmp) { return tmp + 1; }
+template <class T>
+__host__ __device__ __forceinline__ T* split_rhs(T* tmp, int n) {
+  const long m = (long)n + 2;
+  return tmp + m * m * m - 1;
+}
+
 // the level L of the case this block serves in a bucket launch (L itself
 // outside one)
 template <class T>
@@ -62,11 +76,10 @@ __device__ __forceinline__ Lvl<T> rebase(const Lvl<T>& L, const Batch& bt) {
   const CasePtrs& cp = bt.tab[bt_case(bt)];
   Lvl<T> R = L;
   const int l = L.role & 15;
-  const long m = (long)L.n + 2;
   T* tmp = (T*)cp.mg_tmp[l];
   if (L.role & LV_SPLIT) {
-    R.phi = tmp;
-    R.rhs = tmp + m * m * m;
+    R.phi = split_phi(tmp);
+    R.rhs = split_rhs(tmp, L.n);
   } else if (L.role & LV_PP) {
     const long P = (long)L.n + 2 * NPL;
     const long off = (long)(NPL - 1) * (P * P + P + 1);
@@ -2087,8 +2100,8 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
   if (bt.tab) {
-    sp = L.tmp;
-    sr = L.tmp + (long)(L.n + 2) * (L.n + 2) * (L.n + 2);
+    sp = split_phi(L.tmp);
+    sr = split_rhs(L.tmp, L.n);
   }
   const int m = L.n + 2, H = m >> 1;
   const int row = blockIdx.x * SPLIT_ROWS + (threadIdx.x >> 5);
@@ -2120,8 +2133,8 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
   }
   const Lvl<T> L = rebase(L0, bt);
   if (bt.tab) {
-    sp = L.tmp;
-    sr = L.tmp + (long)(L.n + 2) * (L.n + 2) * (L.n + 2);
+    sp = split_phi(L.tmp);
+    sr = split_rhs(L.tmp, L.n);
   }
   const int n = L.n, nh = n >> 1;
   const int h0 = blockIdx.x * 32 * CPT + threadIdx.x;
@@ -2169,6 +2182,91 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
   }
 }
 
+// the same half-sweep two cells at a time, for n a multiple of 4 (the pairs of
+// cells h = 2q, 2q + 1 are aligned, see split_phi), marching through `planes`
+// planes i with the next plane's operands on their way while one is updated
+constexpr int PAIR_MIN_N = 144;
+
+template <class T>
+struct alignas(2 * sizeof(T)) Two {
+  T x, y;
+};
+
+template <class T>
+struct PairIn {   // operands of one pair that its plane adds
+  Two<T> e, s, n, r;
+  T z;
+};
+
+template <class T>
+__global__ void __launch_bounds__(256)
+    k_rbgs_pair(const Lvl<T> L0, T* sp, const T* sr, int color, int planes, int back,
+                const __grid_constant__ ApRecip<T> rt, const Batch bt) {
+  pdl_chain();
+  if (bt_skip(bt)) return;
+  const Lvl<T> L = rebase(L0, bt);
+  if (bt.tab) {
+    sp = split_phi(L.tmp);
+    sr = split_rhs(L.tmp, L.n);
+  }
+  const int n = L.n, q = threadIdx.x;
+  const int j = blockIdx.x * blockDim.y + threadIdx.y;
+  const int seg = back ? bt_gz(bt) - 1 - bt_z(bt) : bt_z(bt);
+  const int iend = min(n, (seg + 1) * planes);
+  int i = seg * planes;
+  if (j >= n) return;
+  const int H = (n + 2) >> 1, tI = (int)L.tI, tJ = (int)L.tJ;
+  const T as = j > 0 ? L.ay : T(0), an = j < n - 1 ? L.ay : T(0);
+  const int pj = 3 * ((j > 0) + (j < n - 1));
+  using V = Two<T>;
+  const long r0 = (long)(j + 1) * tJ + 2 * q;
+  auto vec = [](const T* p) { return *reinterpret_cast<const V*>(p); };
+  // parity pr of a = k+1 of the row's colour; the other colour of a row sits
+  // where the colour of the planes beside it sits, so the pair loaded as the
+  // i+1 neighbour of plane i holds two of the three k neighbours in plane i+1
+  // and the i-1 neighbour in plane i+2
+  auto load = [&](int ii) {
+    PairIn<T> a;
+    const int pr = (ii + j + color) & 1;
+    const long r = (long)(ii + 1) * L.tI + r0;
+    const T* own = sp + r + (pr ? H : 1);
+    a.e = vec(own + tI);
+    a.s = vec(own - tJ);
+    a.n = vec(own + tJ);
+    a.r = vec(sr + r + (pr ? H : 1));
+    a.z = sp[r + (pr ? 0 : H + 2)];          // a-1 of the first cell, a+1 of the second
+    return a;
+  };
+  V w, z;
+  {
+    const int pr = (i + j + color) & 1;
+    const long r = (long)(i + 1) * L.tI + r0;
+    w = vec(sp + r + (pr ? H : 1) - tI);
+    z = vec(sp + r + (pr ? 1 : H));
+  }
+  PairIn<T> cur = load(i);
+  for (; i < iend; ++i) {
+    PairIn<T> nxt = cur;
+    if (i + 1 < iend) nxt = load(i + 1);
+    const int pr = (i + j + color) & 1;
+    const T z0 = pr ? cur.z : z.x, z1 = pr ? z.x : z.y, z2 = pr ? z.y : cur.z;
+    const T aw = i > 0 ? L.ax : T(0), ae = i < n - 1 ? L.ax : T(0);
+    const int pij = 9 * ((i > 0) + (i < n - 1)) + pj;
+    const int k0 = 4 * q + 1 - pr, k1 = k0 + 2;   // k of the two cells
+    const T ab = k0 > 0 ? L.az : T(0), at = k1 < n - 1 ? L.az : T(0);
+    const T ap0 = -(aw + ae + as + an + ab + L.az), ap1 = -(aw + ae + as + an + L.az + at);
+    const T s0 = aw * w.x + ae * cur.e.x + as * cur.s.x + an * cur.n.x + ab * z0 + L.az * z1;
+    const T s1 = aw * w.y + ae * cur.e.y + as * cur.s.y + an * cur.n.y + L.az * z1 + at * z2;
+    V x;
+    x.x = div_by_recip(cur.r.x - s0, ap0, rt.y[pij + (k0 > 0) + 1]);
+    x.y = div_by_recip(cur.r.y - s1, ap1, rt.y[pij + 1 + (k1 < n - 1)]);
+    *reinterpret_cast<V*>(sp + (long)(i + 1) * L.tI + r0 + (pr ? H : 1)) = x;
+    w = z;
+    z = cur.e;
+    cur = nxt;
+  }
+}
+
 // the same half-sweep with the colour's cells of a plane numbered flat
 // (rnh = 1 / cells per half-row), CPT cells a thread
 constexpr int FLAT_MAX_N = 104;
@@ -2183,8 +2281,8 @@ __global__ void __launch_bounds__(MG_TPB)
   }
   const Lvl<T> L = rebase(L0, bt);
   if (bt.tab) {
-    sp = L.tmp;
-    sr = L.tmp + (long)(L.n + 2) * (L.n + 2) * (L.n + 2);
+    sp = split_phi(L.tmp);
+    sr = split_rhs(L.tmp, L.n);
   }
   const int n = L.n, nh = n >> 1;
   const int i = bt_z(bt);
@@ -2241,7 +2339,7 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
   pdl_entry();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
-  if (bt.tab) sp = L.tmp;
+  if (bt.tab) sp = split_phi(L.tmp);
   const int n = L.n, H = (n + 2) >> 1;
   const int row = blockIdx.x * SPLIT_ROWS + (threadIdx.x >> 5);
   if (row >= n * n) return;
@@ -2284,34 +2382,48 @@ static int split_min_n() {
 template <class T>
 static int split_in(const Lvl<T>& L, bool with_rhs, cudaStream_t s) {
   const int m = L.n + 2;
-  T* sp = L.tmp;
-  T* sr = L.tmp + (long)m * m * m;
+  T* sp = split_phi(L.tmp);
+  T* sr = split_rhs(L.tmp, L.n);
   WF_CK(launch_k(k_split_in<T>, (m * m + SPLIT_ROWS - 1) / SPLIT_ROWS, 32 * SPLIT_ROWS, 0, s, L,
                  sp, sr, with_rhs ? 1 : 0));
   WF_CKL("k_split_in");
   return WF_OK;
 }
 
-// the half-sweeps of a relax on the split copies.  A half-row of a level below
-// 104 cells does not fill k_rbgs_split's warps (40 of 64 or 128 lanes at 80^3)
-// and its CTAs are many and small: there the cells are numbered flat, one per
-// thread, two from 86 (the CTAs of one colour are then about one wave).  us per
-// half-sweep in a graph, rows / flat x 1 / flat x 2, FP64: 64^3 2.10 / 1.68 /
-// 1.86, 72^3 2.74 / 2.12 / 2.14, 80^3 2.91 / 2.09 / 2.14, 88^3 3.61 / 2.85 /
-// 2.89, 96^3 4.00 / 3.24 / 3.02, 104^3 3.58 / 3.93 / 3.59, 128^3 4.82 / 6.27 /
-// 5.64.  A shape set for the level (wf_set_launch_shape) takes the rows form.
+// the half-sweeps of a relax on the split copies, in one of three forms.
+//  - Below 104 a half-row does not fill k_rbgs_split's warps (40 of 64 or 128
+//    lanes at 80^3) and its CTAs are many and small: the cells are numbered
+//    flat, one per thread, two from 86 (the CTAs of one colour are then about
+//    one wave).  us per half-sweep in a graph, rows / flat x 1 / flat x 2,
+//    FP64: 64^3 2.10 / 1.68 / 1.86, 72^3 2.74 / 2.12 / 2.14, 80^3 2.91 / 2.09 /
+//    2.14, 88^3 3.61 / 2.85 / 2.89, 96^3 4.00 / 3.24 / 3.02, 104^3 3.58 / 3.93 /
+//    3.59, 128^3 4.82 / 6.27 / 5.64.
+//  - From 144, for n a multiple of 4, pairs marching through planes: loads of
+//    two, three of seven operands from the planes before, the next plane on its
+//    way.  rows / pairs, FP64: 128^3 4.87 / 5.46, 160^3 11.6 / 9.2, 192^3 20.6 /
+//    17.7, 256^3 40.9 / 40.0 (5.0 TB/s of DRAM traffic), 320^3 106 / 78; FP32:
+//    128^3 4.4 / 4.6, 160^3 10.4 / 7.2, 192^3 20.0 / 10.6, 256^3 35.0 / 24.2,
+//    320^3 106 / 47.  From 176 every second half-sweep runs its planes backward
+//    (what the one before touched last is still in L2: 256^3 FP64 41.5 -> 40.0).
+//  - Otherwise, and for a shape set for the level (wf_set_launch_shape), the
+//    rows of k_rbgs_split.
 template <class T>
 static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
-  const int m = L.n + 2, nh = L.n / 2;
-  T* sp = L.tmp;
-  const T* sr = L.tmp + (long)m * m * m;
+  const int n = L.n, nh = n / 2;
+  T* sp = split_phi(L.tmp);
+  const T* sr = split_rhs(L.tmp, n);
   const ApRecip<T> rt = ap_recip(L);
-  const bool flat = L.n < FLAT_MAX_N && !launch_shape_set(SHAPE_SPLIT, L.n);
-  const int cells = L.n > 84 ? 2 : 1;
+  const bool set = launch_shape_set(SHAPE_SPLIT, n);
+  const bool flat = n < FLAT_MAX_N && !set;
+  const bool pair = n >= PAIR_MIN_N && n % 4 == 0 && n <= 1024 && !set &&
+                    (uintptr_t)L.tmp % (2 * sizeof(T)) == 0;
+  const int cells = n > 84 ? 2 : 1;
+  const int planes = n >= 176 ? 4 : 2, prows = std::min(n >= 176 ? 2 : 4, MG_TPB / (n / 4));
   int cpt, rows, one;
-  launch_shape(SHAPE_SPLIT, L.n, &cpt, &rows, &one);   // cpt in {1, 2, 4, 8}, rows <= SPLIT_ROWS
-  const dim3 grid((nh + 32 * cpt - 1) / (32 * cpt), (L.n + rows - 1) / rows, L.n);
-  const dim3 fgrid((L.n * nh + MG_TPB * cells - 1) / (MG_TPB * cells), 1, L.n);
+  launch_shape(SHAPE_SPLIT, n, &cpt, &rows, &one);   // cpt in {1, 2, 4, 8}, rows <= SPLIT_ROWS
+  const dim3 grid((nh + 32 * cpt - 1) / (32 * cpt), (n + rows - 1) / rows, n);
+  const dim3 fgrid((n * nh + MG_TPB * cells - 1) / (MG_TPB * cells), 1, n);
+  const dim3 pgrid((n + prows - 1) / std::max(1, prows), 1, (n + planes - 1) / planes);
   auto kern = cpt == 8   ? k_rbgs_split<T, 8>
               : cpt == 4 ? k_rbgs_split<T, 4>
               : cpt == 2 ? k_rbgs_split<T, 2>
@@ -2319,11 +2431,14 @@ static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
   auto kflat = cells == 2 ? k_rbgs_flat<T, 2> : k_rbgs_flat<T, 1>;
   for (int h = 0; h < 2 * nsweeps; ++h) {
     // from the second half-sweep on, the launch ahead is a half-sweep
-    const int pre = h > 0 ? 1 : 0;
+    const int pre = h > 0 ? 1 : 0, color = h & 1, back = n >= 176 ? color : 0;
     if (flat)
-      WF_CK(launch_chain(kflat, fgrid, MG_TPB, 0, s, L, sp, sr, h & 1, pre, 1.0f / (float)nh, rt));
+      WF_CK(launch_chain(kflat, fgrid, MG_TPB, 0, s, L, sp, sr, color, pre, 1.0f / (float)nh, rt));
+    else if (pair)
+      WF_CK(launch_chain(k_rbgs_pair<T>, pgrid, dim3(n / 4, prows), 0, s, L, sp, sr, color, planes,
+                         back, rt));
     else
-      WF_CK(launch_chain(kern, grid, dim3(32, rows), 0, s, L, sp, sr, h & 1, pre, rt));
+      WF_CK(launch_chain(kern, grid, dim3(32, rows), 0, s, L, sp, sr, color, pre, rt));
     WF_CKL("k_rbgs_split");
   }
   return WF_OK;
@@ -2333,7 +2448,7 @@ static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
 template <class T>
 static int split_out(const Lvl<T>& L, cudaStream_t s) {
   WF_CK(launch_k(k_split_out<T>, (L.n * L.n + SPLIT_ROWS - 1) / SPLIT_ROWS, 32 * SPLIT_ROWS, 0,
-                 s, L, (const T*)L.tmp));
+                 s, L, (const T*)split_phi(L.tmp)));
   WF_CKL("k_split_out");
   return WF_OK;
 }
@@ -2355,9 +2470,8 @@ template <class T>
 static Lvl<T> split_view(const Lvl<T>& L) {
   Lvl<T> V = L;
   V.role = L.role | LV_SPLIT;
-  const long m = (long)L.n + 2;
-  V.phi = L.tmp;
-  V.rhs = L.tmp + m * m * m;
+  V.phi = split_phi(L.tmp);
+  V.rhs = split_rhs(L.tmp, L.n);
   V.sI = L.tI;
   V.sJ = L.tJ;
   V.split = 1;
