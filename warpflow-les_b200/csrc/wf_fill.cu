@@ -260,7 +260,7 @@ static int program(int kind, int n, double val, const double* valp, int phase, F
 // Table entries are (dst, code): dst the cell's offset in the field; code
 // bit 0 set: a constant (bits 2.. = 0 for 0.0, 1 for the fill's value),
 // else bits 2.. = the source offset; bit 1 set: negate.
-constexpr int ONE_GMAX = 4;         // cells of one group (2 or 3 occur)
+constexpr int ONE_GMAX = 6;         // cells of one group (up to 5 at edges 4 and 5, 3 from 6)
 constexpr int ONE_NMAX = 256;       // largest n served by one-launch fills
 
 struct OneProg {
