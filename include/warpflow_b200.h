@@ -327,9 +327,9 @@ typedef struct wf_stepper wf_stepper;
  * after its predecessor finished, which frees SMs for other streams when
  * many steppers run concurrently (ensembles, serving). */
 #define WF_STEP_SERIAL 2
-/* With WF_STEP_SERIAL: the half-sweeps of the multigrid still launch with
- * programmatic dependent launch (each computes its indices and reads its
- * right-hand side while the one before it runs). */
+/* With WF_STEP_SERIAL: the ghost fills and the multigrid's kernels still launch
+ * with programmatic dependent launch (each computes its indices and reads what
+ * was complete earlier while the one before it runs). */
 #define WF_STEP_CHAIN 8
 WF_API int wf_stepper_create(const wf_case* c, int32_t mode, wf_stepper** out);
 /* One FlowSolver.step(): enqueue the step on `stream`.  No host sync. */

@@ -41,7 +41,7 @@ extern thread_local long g_launches;
 inline int64_t padded(int n) { return (int64_t)n + 2 * NPL; }
 
 // programmatic dependent launch on (default) or off (WF_PDL=0, WF_STEP_SERIAL);
-// chain: for the half-sweeps, which WF_STEP_CHAIN keeps on
+// chain: for the kernels in pdl_chain order, which WF_STEP_CHAIN keeps on
 bool pdl_enabled(bool chain = false);
 
 // one thread per cell of an ni x nj x nk box: CTAs of 32 (k) x 8 (j) threads,
@@ -125,7 +125,7 @@ inline cudaError_t launch_k(void (*kernel)(ExpTypes...), dim3 grid, dim3 block, 
   }
 }
 
-// launch_k for the kernels of a half-sweep chain (pdl_chain)
+// launch_k for the kernels in pdl_chain order
 template <typename K, typename... ActTypes>
 inline cudaError_t launch_chain(K kernel, dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                                 ActTypes&&... args) {

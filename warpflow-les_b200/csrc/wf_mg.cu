@@ -199,21 +199,26 @@ static int launch_rbgs(const Lvl<T>& L, int color, bool pre, cudaStream_t s) {
 }
 
 // restriction (multigrid.py:93-119): rhs_c = 1/8 sum of the 8 fine residuals;
-// also zeroes the coarse level's phi, ring included
+// also zeroes the coarse level's phi, ring included.  A short launch at coarse
+// sizes: the indices and, with pre, the eight fine rhs values come ahead of the
+// wait.  This, the same in the prolongations (fine phi) and the coarse-operator
+// kernels, all in the chain, with k_cop_gemm's four representatives to a warp:
+// us per step at 32^3 417 -> 408, 80^3 702 -> 695, 96^3 995 -> 965, 128^3 mixed
+// 1520 -> 1500, 256^3 FP64 unchanged (its transfers are bandwidth)
 template <class T>
 __global__ void __launch_bounds__(MG_TPB) k_restrict(const Lvl<T> F0, T* rhs_c, Lvl<T> C0,
-                                                     const Batch bt) {
-  pdl_entry();
-  if (bt_skip(bt)) return;
+                                                     int pre, const Batch bt) {
+  if (bt.tab) {
+    pdl_chain();
+    if (bt_skip(bt)) return;
+  }
   const Lvl<T> F = rebase(F0, bt);
   const Lvl<T> C = rebase(C0, bt);
   if (bt.tab) rhs_c = const_cast<T*>(C.rhs);
   const int nc = C.n, n = F.n;
   {  // one thread per cell: x = ck (runs of 32), y = cj (groups of 8), z = ci
-    const int kx_ = blockIdx.x * 32 + threadIdx.x, jy_ = blockIdx.y * 8 + threadIdx.y;
-    if (kx_ >= nc || jy_ >= nc) return;
-    const int ck = kx_;
-    const int cj = jy_;
+    const int ck = blockIdx.x * 32 + threadIdx.x, cj = blockIdx.y * 8 + threadIdx.y;
+    const bool on = ck < nc && cj < nc;
     const int ci = bt_z(bt);
     // the fine phi values the 8 residuals read -- the 2x2x2 block and its
     // face neighbours, P[a][b][c] at fine cell (2ci-1+a, 2cj-1+b, 2ck-1+c)
@@ -224,6 +229,19 @@ __global__ void __launch_bounds__(MG_TPB) k_restrict(const Lvl<T> F0, T* rhs_c, 
 #pragma unroll
     for (int q = 0; q < 4; ++q) kp[q] = F.split ? spos(k0 + q, H) : (k0 + q);
     const T* p = F.phi;
+    T r8[2][2][2];   // pre: the fine rhs was complete before the launch ahead (pdl_chain)
+    if (pre && on) {
+#pragma unroll
+      for (int di = 0; di < 2; ++di)
+#pragma unroll
+        for (int dj = 0; dj < 2; ++dj)
+#pragma unroll
+          for (int dk = 0; dk < 2; ++dk)
+            r8[di][dj][dk] = __ldcg(F.rhs + (long)(i0 + di + 1) * F.sI +
+                                    (long)(j0 + dj + 1) * F.sJ + kp[1 + dk]);
+    }
+    if (!bt.tab) pdl_chain();
+    if (!on) return;
     T P[4][4][4];
 #pragma unroll
     for (int a = 0; a < 4; ++a)
@@ -246,7 +264,8 @@ __global__ void __launch_bounds__(MG_TPB) k_restrict(const Lvl<T> F0, T* rhs_c, 
           const T ab = k > 0 ? F.az : T(0), at = k < n - 1 ? F.az : T(0);
           const T ap = -(aw + ae + as + an + ab + at);
           const int a = 1 + di, b = 1 + dj, q = 1 + dk;
-          const T r = F.rhs[(long)(i + 1) * F.sI + (long)(j + 1) * F.sJ + kp[q]];
+          const T r = pre ? r8[di][dj][dk]
+                          : F.rhs[(long)(i + 1) * F.sI + (long)(j + 1) * F.sJ + kp[q]];
           const T res = r - (aw * P[a - 1][b][q] + ae * P[a + 1][b][q] + as * P[a][b - 1][q] +
                              an * P[a][b + 1][q] + ab * P[a][b][q - 1] + at * P[a][b][q + 1] +
                              ap * P[a][b][q]);
@@ -269,7 +288,7 @@ __global__ void __launch_bounds__(MG_TPB) k_restrict(const Lvl<T> F0, T* rhs_c, 
 // zero a whole array (in a bucket launch: field slot `fid` of every case)
 template <class T>
 __global__ void k_zero(T* a, long cnt, int fid, const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;
   if (bt.tab) a = (T*)bt.tab[bt_case(bt)].fld[fid];
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < cnt;
@@ -280,7 +299,7 @@ __global__ void k_zero(T* a, long cnt, int fid, const Batch bt) {
 // zero a (n+2)^3 block embedded with strides (sI, sJ)
 template <class T>
 __global__ void k_zero_strided(T* a, int m, long sI, long sJ) {
-  pdl_entry();
+  pdl_chain();
   const long tot = (long)m * m * m;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < tot;
        t += (long)gridDim.x * blockDim.x) {
@@ -294,17 +313,22 @@ __global__ void k_zero_strided(T* a, int m, long sI, long sJ) {
 // prolongation (multigrid.py:122-146) + the ring refill that follows it
 template <class T>
 __global__ void __launch_bounds__(MG_TPB) k_prolong(const Lvl<T> C0, Lvl<T> F0, const Batch bt) {
-  pdl_entry();
-  if (bt_skip(bt)) return;
+  if (bt.tab) {
+    pdl_chain();
+    if (bt_skip(bt)) return;
+  }
   const Lvl<T> C = rebase(C0, bt);
   const Lvl<T> F = rebase(F0, bt);
   const int n = F.n;
   {  // one thread per cell: x = k (runs of 32), y = j (groups of 8), z = i
-    const int kx_ = blockIdx.x * 32 + threadIdx.x, jy_ = blockIdx.y * 8 + threadIdx.y;
-    if (kx_ >= n || jy_ >= n) return;
-    const int k = kx_;
-    const int j = jy_;
+    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
+    const bool on = k < n && j < n;
     const int i = bt_z(bt);
+    const long c = lid(F, i + 1, j + 1, k + 1);
+    // written before the restriction out of this level (pdl_chain)
+    const T old = on ? __ldcg(F.phi + c) : T(0);
+    if (!bt.tab) pdl_chain();
+    if (!on) return;
     const int c0x = (i % 2 == 0) ? i / 2 - 1 : i / 2;
     const T wx0 = (i % 2 == 0) ? T(0.25) : T(0.75);
     const int c0y = (j % 2 == 0) ? j / 2 - 1 : j / 2;
@@ -325,8 +349,7 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong(const Lvl<T> C0, Lvl<T> F0, 
         }
       }
     }
-    const long c = lid(F, i + 1, j + 1, k + 1);
-    const T x = F.phi[c] + acc;
+    const T x = old + acc;
     F.phi[c] = x;
     if (!F.split) ring_mirror(F, i, j, k, c, x);
   }
@@ -343,14 +366,31 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong(const Lvl<T> C0, Lvl<T> F0, 
 // thread only, and ring_mirror writes ring cells, which are never loaded.
 template <class T>
 __global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0, const Batch bt) {
-  pdl_entry();
-  if (bt_skip(bt)) return;
+  if (bt.tab) {
+    pdl_chain();
+    if (bt_skip(bt)) return;
+  }
   const Lvl<T> C = rebase(C0, bt);
   const Lvl<T> F = rebase(F0, bt);
   const int nc = C.n;
   const int ck = blockIdx.x * 32 + threadIdx.x, cj = blockIdx.y * 8 + threadIdx.y;
-  if (ck >= nc || cj >= nc) return;
+  const bool on = ck < nc && cj < nc;
   const int ci = bt_z(bt);
+  // the fine level was last written before the restriction out of it, at least
+  // two launches ahead (pdl_chain)
+  long fc[2][2][2];
+  T fv[2][2][2];
+#pragma unroll
+  for (int pi = 0; pi < 2; ++pi)
+#pragma unroll
+    for (int pj = 0; pj < 2; ++pj)
+#pragma unroll
+      for (int pk = 0; pk < 2; ++pk) {
+        fc[pi][pj][pk] = lid(F, 2 * ci + pi + 1, 2 * cj + pj + 1, 2 * ck + pk + 1);
+        fv[pi][pj][pk] = on ? __ldcg(F.phi + fc[pi][pj][pk]) : T(0);
+      }
+  if (!bt.tab) pdl_chain();
+  if (!on) return;
   const int Hc = (nc + 2) >> 1;
   long kq[3];
 #pragma unroll
@@ -363,17 +403,6 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0,
 #pragma unroll
       for (int q = 0; q < 3; ++q)
         Q[a][b][q] = C.phi[(long)(ci + a) * C.sI + (long)(cj + b) * C.sJ + kq[q]];
-  long fc[2][2][2];
-  T fv[2][2][2];
-#pragma unroll
-  for (int pi = 0; pi < 2; ++pi)
-#pragma unroll
-    for (int pj = 0; pj < 2; ++pj)
-#pragma unroll
-      for (int pk = 0; pk < 2; ++pk) {
-        fc[pi][pj][pk] = lid(F, 2 * ci + pi + 1, 2 * cj + pj + 1, 2 * ck + pk + 1);
-        fv[pi][pj][pk] = F.phi[fc[pi][pj][pk]];
-      }
 #pragma unroll
   for (int pi = 0; pi < 2; ++pi)
 #pragma unroll
@@ -411,7 +440,7 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0,
 // After the last sweep the interior and the face rings go back to global.
 template <class T>
 __global__ void __launch_bounds__(1024) k_relax_smem(Lvl<T> L0, int nsweeps, const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -530,7 +559,7 @@ __global__ void __launch_bounds__(CoarseShape<NC>::THREADS) k_coarse_cols(Lvl<T>
                                                                            T* unit_out,
                                                                            const int* unit_ids,
                                                                            const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
   constexpr int H = NC / 2;
@@ -668,7 +697,7 @@ struct ClusterShape {
 template <class T, int NC, int NCL>
 __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     k_coarse_cluster(Lvl<T> L, int nsweeps) {
-  pdl_entry();
+  pdl_chain();
   using S = ClusterShape<NC, NCL>;
   constexpr int H = S::H, HALF = S::HALF, GROUP = S::GROUP, PL = S::PL, C = S::C;
   namespace cg = cooperative_groups;
@@ -861,7 +890,7 @@ constexpr int MBAR_WAIT_TRIES = 1 << 22;
 template <class T, int NC, int NCL, bool EXACT>
 __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     k_coarse_p2p(Lvl<T> L, int nsweeps, int wmode) {
-  pdl_entry();
+  pdl_chain();
   using S = ClusterShape<NC, NCL>;
   constexpr int H = S::H, HALF = S::HALF, GROUP = S::GROUP, PL = S::PL, C = S::C;
   namespace cg = cooperative_groups;
@@ -1173,7 +1202,7 @@ __device__ __forceinline__ void cheb_cols(const double* __restrict__ oth, double
 template <int NC, int NCL>
 __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     k_coarse_cheb(Lvl<double> L0, const __grid_constant__ ChebCoef C, int wmode, const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;   // the case's whole cluster
   const Lvl<double> L = rebase(L0, bt);
   using T = double;
@@ -1423,7 +1452,7 @@ struct TbShape {
 template <class T, int NC, int NCL>
 __global__ void __launch_bounds__(TbShape<NC, NCL>::THREADS)
     k_coarse_tb(Lvl<T> L, int nsweeps, int wmode) {
-  pdl_entry();
+  pdl_chain();
   using S = TbShape<NC, NCL>;
   constexpr int H = S::H, HALF = S::HALF, GROUP = S::GROUP, PL = S::PL, C = S::C;
   constexpr int SIDE = S::SIDE;
@@ -1649,7 +1678,7 @@ static int try_coarse_tb(const Lvl<T>& L, int nsweeps, cudaStream_t s, int* rc) 
 // equal the mathematical S to rounding, so the relax agrees with the
 // sweeps to rounding.
 constexpr int COP_GMAX = 24;
-static_assert(COP_GMAX <= 32, "k_cop_gemm writes symmetry q from lane q");
+static_assert(COP_GMAX == 24, "k_cop_gemm adds 4 x 12 values over the lanes of a warp");
 
 static bool cop_size_ok(int nc) {
   return nc == 4 || nc == 8 || nc == 12 || nc == 16 || nc == 20 || nc == 24;
@@ -1680,7 +1709,7 @@ struct CopPlan {
   }
 };
 
-constexpr int COP_RB = 16;  // representatives per CTA of k_cop_gemm (2 per warp)
+constexpr int COP_RB = 16;  // representatives per CTA of k_cop_gemm (4 per two warps)
 constexpr int COP_KS = 8;   // slices of the B cells (the product's sum) per output
 
 // per-case scratch of the operator product: the permuted copies of v_B
@@ -1802,7 +1831,7 @@ template <class T>
 __global__ void __launch_bounds__(256) k_cop_vg(const Lvl<T> L0, T* V,
                                                 const __grid_constant__ CopSyms G,
                                                 const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
   if (bt.tab) V = (T*)bt.tab[bt_case(bt)].mg_cop_part;
@@ -1853,20 +1882,24 @@ template <> struct Vec2<float> { using type = float2; };
 
 // Y_s[x][g] = sum over the s-th slice of B cells u of C[x][u] * V[g][u]:
 // a CTA takes COP_RB representatives x and one slice, and first copies the
-// slice of every permuted copy V[g] into shared memory (each CTA reads it
-// once from L2; the operator rows are read once in all) -- COP_SB loads per
-// thread issued before any is stored, a few rounds of L2 latency instead of
-// one per element (the 20^3 relax 28.8 -> 24.7 us); warp w takes the
-// representatives x0 + 2w, x0 + 2w + 1 and every symmetry; lanes step
-// through the slice two cells at a time (2-vector loads), each summing its
-// cells in ascending order, then the lanes are added by a butterfly (fixed
-// order)
-constexpr int COP_SB = 16;   // staging loads in flight per thread
+// slice of every permuted copy V[g] into shared memory (all copies in flight at
+// once, a warp per copy).  Warp w takes four representatives and half of the
+// symmetries: what bounds the product is the reading of the slices from shared
+// memory, and a value read serves four representatives.  Lanes step through the
+// slice two cells at a time (2-vector loads), each summing its cells in
+// ascending order; then the lanes are added in the order of a butterfly (16, 8,
+// 4, 2, 1), each step halving the values a lane still carries instead of
+// repeating every sum in both halves.
+template <class T>
+__device__ __forceinline__ void cop_copy(void* d, const void* s) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(smem_u32(d)), "l"(s),
+               "n"(2 * sizeof(T)) : "memory");
+}
 
 template <class T>
 __global__ void __launch_bounds__(256) k_cop_gemm(const T* C, const T* V, T* Y, int nrep,
                                                   int M, int ng, const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;
   if (bt.tab) {
     V = (const T*)bt.tab[bt_case(bt)].mg_cop_part;
@@ -1876,72 +1909,67 @@ __global__ void __launch_bounds__(256) k_cop_gemm(const T* C, const T* V, T* Y, 
   extern __shared__ __align__(16) unsigned char cop_smem[];
   V2* sv = reinterpret_cast<V2*>(cop_smem);   // [ng][nh]: this slice of every V[g]
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int x0 = blockIdx.x * COP_RB, s = blockIdx.y;
+  const int s = blockIdx.y;
   const int per = (((M + COP_KS - 1) / COP_KS) + 1) & ~1;   // even: 2-vector aligned
   const int h0 = s * per / 2, h1 = min(M, s * per + per) / 2;   // 2-vector range
   const int nh = max(0, h1 - h0);
-  const int nv = ng * nh;
-  for (int t0 = threadIdx.x; t0 < nv; t0 += blockDim.x * COP_SB) {
-    V2 buf[COP_SB];
-#pragma unroll
-    for (int b = 0; b < COP_SB; ++b) {
-      const int t = t0 + b * blockDim.x;
-      if (t < nv) {
-        const int g = t / nh, h = t - g * nh;
-        buf[b] = reinterpret_cast<const V2*>(V + (long)g * M)[h0 + h];
-      }
-    }
-#pragma unroll
-    for (int b = 0; b < COP_SB; ++b) {
-      const int t = t0 + b * blockDim.x;
-      if (t < nv) sv[t] = buf[b];
-    }
+  for (int g = w; g < ng; g += 8) {
+    const V2* src = reinterpret_cast<const V2*>(V + (long)g * M) + h0;
+    for (int h = lane; h < nh; h += 32) cop_copy<T>(sv + g * nh + h, src + h);
   }
+  constexpr int NR = 4, NG = COP_GMAX / 2;    // representatives and symmetries of a warp
+  const int r0 = blockIdx.x * COP_RB + (w >> 1) * NR, g0 = (w & 1) * NG;
+  const V2* cp[NR];
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+    cp[r] = reinterpret_cast<const V2*>(C + (long)min(r0 + r, nrep - 1) * M);
+  T acc[NR * NG];
+#pragma unroll
+  for (int q = 0; q < NR * NG; ++q) acc[q] = T(0);
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  const int r0 = x0 + 2 * w;
-  T acc[2][COP_GMAX];
-#pragma unroll
-  for (int q = 0; q < COP_GMAX; ++q) acc[0][q] = acc[1][q] = T(0);
-  if (r0 < nrep) {
-    const V2* c0p = reinterpret_cast<const V2*>(C + (long)r0 * M);
-    const V2* c1p = reinterpret_cast<const V2*>(C + (long)min(r0 + 1, nrep - 1) * M);
+  if (r0 >= nrep) return;
 #pragma unroll 1
-    for (int h = h0 + lane; h < h1; h += 32) {
-      const V2 c0 = c0p[h], c1 = c1p[h];
-      const V2* vh = sv + (h - h0);
+  for (int h = h0 + lane; h < h1; h += 32) {
+    V2 cv[NR];
 #pragma unroll
-      for (int q = 0; q < COP_GMAX; ++q) {
-        if (q < ng) {
-          const V2 v = vh[q * nh];
-          acc[0][q] = fma(c0.x, v.x, acc[0][q]);
-          acc[0][q] = fma(c0.y, v.y, acc[0][q]);
-          acc[1][q] = fma(c1.x, v.x, acc[1][q]);
-          acc[1][q] = fma(c1.y, v.y, acc[1][q]);
+    for (int r = 0; r < NR; ++r) cv[r] = cp[r][h];
+    const V2* vh = sv + g0 * nh + (h - h0);
+#pragma unroll
+    for (int q = 0; q < NG; ++q) {
+      if (g0 + q < ng) {
+        const V2 v = vh[q * nh];
+#pragma unroll
+        for (int r = 0; r < NR; ++r) {
+          acc[r * NG + q] = fma(cv[r].x, v.x, acc[r * NG + q]);
+          acc[r * NG + q] = fma(cv[r].y, v.y, acc[r * NG + q]);
         }
       }
     }
   }
+  // 48 values over 32 lanes: after the steps 16, 8, 4, 2 a lane holds the three
+  // values 24 b4 + 12 b3 + 6 b2 + 3 b1 .. + 2 (b: bits of the lane)
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
+  for (int o = 16, half = 24; o > 1; o >>= 1, half >>= 1) {
+    const bool hi = (lane & o) != 0;
 #pragma unroll
-    for (int q = 0; q < COP_GMAX; ++q) {
-      T y = acc[r][q];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
-      acc[r][q] = y;
+    for (int q = 0; q < 24; ++q) {
+      if (q < half) {
+        const T send = hi ? acc[q] : acc[q + half], keep = hi ? acc[q + half] : acc[q];
+        acc[q] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      }
     }
-  // lane q writes symmetry q of both representatives
-  T y0 = T(0), y1 = T(0);
-#pragma unroll
-  for (int q = 0; q < COP_GMAX; ++q)
-    if (lane == q) {
-      y0 = acc[0][q];
-      y1 = acc[1][q];
-    }
-  if (lane < ng) {
-    if (r0 < nrep) Y[((long)s * nrep + r0) * COP_GMAX + lane] = y0;
-    if (r0 + 1 < nrep) Y[((long)s * nrep + r0 + 1) * COP_GMAX + lane] = y1;
   }
+#pragma unroll
+  for (int q = 0; q < 3; ++q) acc[q] += __shfl_xor_sync(0xffffffffu, acc[q], 1);
+  if (lane & 1) return;
+  const int at = 24 * ((lane >> 4) & 1) + 12 * ((lane >> 3) & 1) + 6 * ((lane >> 2) & 1) +
+                 3 * ((lane >> 1) & 1);
+  const int r = at / NG, q0 = at - r * NG;    // three values of one representative
+  if (r0 + r >= nrep) return;
+#pragma unroll
+  for (int q = 0; q < 3; ++q)
+    if (g0 + q0 + q < ng) Y[((long)s * nrep + r0 + r) * COP_GMAX + g0 + q0 + q] = acc[q];
 }
 
 // shared memory of k_cop_gemm: the slice of every permuted copy
@@ -1957,14 +1985,14 @@ static size_t cop_gemm_smem(int M, int ng) {
 template <class T>
 __global__ void __launch_bounds__(256) k_cop_out(const T* Y, const int* prod, int nrep,
                                                  Lvl<T> L0, const Batch bt) {
-  pdl_entry();
+  const int M0 = L0.n * L0.n * L0.n / 2, o = blockIdx.x * 256 + threadIdx.x;
+  const int pv = o < M0 ? prod[o] : 0;     // the operator is constant
+  pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
   const int n = L.n, M = n * n * n / 2;
   if (bt.tab) Y = (const T*)bt.tab[bt_case(bt)].mg_cop_part + (long)COP_GMAX * M;
-  const int o = blockIdx.x * 256 + threadIdx.x;
   if (o >= M) return;
-  const int pv = prod[o];
   const long at = (long)(pv >> 5) * COP_GMAX + (pv & 31);
   T y = Y[at];
 #pragma unroll
@@ -1987,16 +2015,17 @@ static int apply_coarse_op(const Lvl<T>& L, const T* op, T* part, cudaStream_t s
   T* V = part;
   T* Y = part + (long)COP_GMAX * P.M;
   const int* prod = reinterpret_cast<const int*>(op + (long)P.nrep * P.M) + P.nrep;
-  WF_CK(launch_k(k_cop_vg<T>, (P.M + 31) / 32, 256, 0, s, L, V, P.G));
+  WF_CK(launch_chain(k_cop_vg<T>, (P.M + 31) / 32, 256, 0, s, L, V, P.G));
   WF_CKL("k_cop_vg");
   const size_t sm = cop_gemm_smem<T>(P.M, P.G.ng);
   WF_CK(cudaFuncSetAttribute(k_cop_gemm<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-  WF_CK(launch_k(k_cop_gemm<T>, dim3((P.nrep + COP_RB - 1) / COP_RB, COP_KS), 256, sm, s, op,
+  WF_CK(launch_chain(k_cop_gemm<T>, dim3((P.nrep + COP_RB - 1) / COP_RB, COP_KS), 256, sm, s, op,
                  (const T*)V, Y, P.nrep, P.M, P.G.ng));
   WF_CKL("k_cop_gemm");
-  WF_CK(launch_k(k_cop_out<T>, (P.M + 255) / 256, 256, 0, s, (const T*)Y, prod, P.nrep, L));
+  WF_CK(launch_chain(k_cop_out<T>, (P.M + 255) / 256, 256, 0, s, (const T*)Y, prod, P.nrep, L));
   WF_CKL("k_cop_out");
-  for (int color = 0; color < 2; ++color) WF_TRY(launch_rbgs(L, color, color > 0, s));
+  // the rhs was written before k_cop_vg
+  for (int color = 0; color < 2; ++color) WF_TRY(launch_rbgs(L, color, true, s));
   return WF_OK;
 }
 
@@ -2096,7 +2125,7 @@ constexpr int SPLIT_ROWS = 8;  // rows (one warp each) per CTA
 template <class T>
 __global__ void __launch_bounds__(32 * SPLIT_ROWS)
     k_split_in(const Lvl<T> L0, T* sp, T* sr, int with_rhs, const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
   if (bt.tab) {
@@ -2336,7 +2365,7 @@ __global__ void __launch_bounds__(MG_TPB)
 template <class T>
 __global__ void __launch_bounds__(32 * SPLIT_ROWS)
     k_split_out(const Lvl<T> L0, const T* sp, const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
   if (bt.tab) sp = split_phi(L.tmp);
@@ -2407,8 +2436,9 @@ static int split_in(const Lvl<T>& L, bool with_rhs, cudaStream_t s) {
 //    (what the one before touched last is still in L2: 256^3 FP64 41.5 -> 40.0).
 //  - Otherwise, and for a shape set for the level (wf_set_launch_shape), the
 //    rows of k_rbgs_split.
+// rhs_ready: the split rhs was complete before the launch ahead of the first one
 template <class T>
-static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
+static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = false) {
   const int n = L.n, nh = n / 2;
   T* sp = split_phi(L.tmp);
   const T* sr = split_rhs(L.tmp, n);
@@ -2431,7 +2461,7 @@ static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
   auto kflat = cells == 2 ? k_rbgs_flat<T, 2> : k_rbgs_flat<T, 1>;
   for (int h = 0; h < 2 * nsweeps; ++h) {
     // from the second half-sweep on, the launch ahead is a half-sweep
-    const int pre = h > 0 ? 1 : 0, color = h & 1, back = n >= 176 ? color : 0;
+    const int pre = h > 0 || rhs_ready ? 1 : 0, color = h & 1, back = n >= 176 ? color : 0;
     if (flat)
       WF_CK(launch_chain(kflat, fgrid, MG_TPB, 0, s, L, sp, sr, color, pre, 1.0f / (float)nh, rt));
     else if (pair)
@@ -2482,7 +2512,7 @@ static Lvl<T> split_view(const Lvl<T>& L) {
 // prolongation out of this level reads them)
 template <class T>
 __global__ void __launch_bounds__(256) k_split_ring(const Lvl<T> V0, const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> V = rebase(V0, bt);
   const int n = V.n;
@@ -2540,7 +2570,7 @@ __global__ void __launch_bounds__(SweepTile<TJ, TK>::THREADS)
     k_sweep2(const T* src, long sIs, long sJs, T* dst, long sId,
              long sJd, const T* rhs, long sIr, long sJr, int n, T ax, T ay,
              T az, int seg, int write_ring) {
-  pdl_entry();
+  pdl_chain();
   using W = SweepTile<TJ, TK>;
   constexpr int WJ = W::WJ, WK = W::WK, WH = W::WH, PLANE = W::PLANE, NT = W::THREADS;
   constexpr int HALF = WJ * WH;                // one parity of a plane
@@ -2735,7 +2765,7 @@ __device__ __forceinline__ void grid_barrier(unsigned* gbar, unsigned nblocks, i
 
 template <class T>
 __global__ void __launch_bounds__(MG_TPB) k_relax_persist(const Lvl<T> L, int nsweeps) {
-  pdl_entry();
+  pdl_chain();
   const int n = L.n;
   const int nh = (n + 1) >> 1;
   const long tot = (long)n * n * nh;
@@ -2849,7 +2879,7 @@ int wait_probe(unsigned* gbar, int* err, int kind, int tries, cudaStream_t s) {
 // max |rhs - A phi| over a level (tests/test_mg.py:16-32)
 __global__ void k_resmax(const Lvl<double> L, double* out, unsigned int* ticket,
                          unsigned long long* acc) {
-  pdl_entry();
+  pdl_chain();
   __shared__ double sm[32];
   const int n = L.n;
   double m = 0.0;
@@ -2958,7 +2988,7 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
     return WF_OK;
   }
   for (int sw = 0; sw < nsweeps; ++sw) {
-    WF_TRY(launch_rbgs(L, 0, sw > 0, s));
+    WF_TRY(launch_rbgs(L, 0, sw > 0 || rhs_ready, s));
     WF_TRY(launch_rbgs(L, 1, true, s));
   }
   return WF_OK;
@@ -2991,8 +3021,9 @@ static int vcycle(std::vector<Lvl<T>>& lv, const wf_case& c, cudaStream_t s,
   for (int l = 0; l < L; ++l) {
     if (l > 0) {
       Lvl<T>& C = vw[l];
-      WF_CK(launch_k(k_restrict<T>, cells3(C.n, C.n, C.n), cell_block(), 0, s,
-          vw[l - 1], const_cast<T*>(C.rhs), C));
+      // the finer level's sweeps lie between its rhs and this launch
+      WF_CK(launch_chain(k_restrict<T>, cells3(C.n, C.n, C.n), cell_block(), 0, s, vw[l - 1],
+                         const_cast<T*>(C.rhs), C, c.n_pre > 0 ? 1 : 0));
       WF_CKL("k_restrict");
     } else if (res[0] && !split0_in) {
       WF_TRY(split_in(lv[0], !rhs0_ready, s));
@@ -3010,18 +3041,18 @@ static int vcycle(std::vector<Lvl<T>>& lv, const wf_case& c, cudaStream_t s,
     // fine levels from 64: one thread per coarse cell (fewer loads); smaller
     // ones keep one thread per fine cell (more threads in flight)
     if (lv[l].n >= 64 && (lv[l].n & 1) == 0) {
-      WF_CK(launch_k(k_prolong8<T>, cells3(lv[l + 1].n, lv[l + 1].n, lv[l + 1].n), cell_block(),
+      WF_CK(launch_chain(k_prolong8<T>, cells3(lv[l + 1].n, lv[l + 1].n, lv[l + 1].n), cell_block(),
                      0, s, vw[l + 1], vw[l]));
       WF_CKL("k_prolong8");
     } else {
-      WF_CK(launch_k(k_prolong<T>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s,
+      WF_CK(launch_chain(k_prolong<T>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s,
                      vw[l + 1], vw[l]));
       WF_CKL("k_prolong");
     }
     if (res[l]) {
-      WF_TRY(split_sweeps(lv[l], c.n_post, s));
+      WF_TRY(split_sweeps(lv[l], c.n_post, s, c.n_pre > 0));
       if (l > 0) {
-        WF_CK(launch_k(k_split_ring<T>, (6 * lv[l].n * lv[l].n + 255) / 256, 256, 0, s, vw[l]));
+        WF_CK(launch_chain(k_split_ring<T>, (6 * lv[l].n * lv[l].n + 255) / 256, 256, 0, s, vw[l]));
         WF_CKL("k_split_ring");
       } else if (!split0_keep) {
         WF_TRY(split_out(lv[0], s));
@@ -3109,7 +3140,7 @@ __device__ __forceinline__ void zero_with_ring(const Lvl<float>& L, int n, int i
 // Lf: the FP32 level 0 (its own arrays, or with LV_SPLIT its split copies)
 __global__ void __launch_bounds__(MG_TPB) k_defect(const Lvl<double> F0, const Lvl<float> Lf0,
                                                    const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<double> F = rebase(F0, bt);
   const Lvl<float> Lf = rebase(Lf0, bt);
@@ -3128,7 +3159,7 @@ __global__ void __launch_bounds__(MG_TPB) k_defect(const Lvl<double> F0, const L
 // what copying it back would have left in the level's own array: the face
 // ring the value of the real cell next to it, edges and corners zero.
 __global__ void k_correct(const Lvl<double> F0, const Lvl<float> Lf0, const Batch bt) {
-  pdl_entry();
+  pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<double> F = rebase(F0, bt);
   const Lvl<float> Lf = rebase(Lf0, bt);
@@ -3344,7 +3375,7 @@ int mg_coarse_solve_pair(const wf_case& c, double* phi, const double* rhs, cudaS
 }
 
 __global__ void k_refill(Lvl<double> L) {
-  pdl_entry();
+  pdl_chain();
   const int n = L.n;
   const long tot = (long)n * n;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < tot;
@@ -3491,14 +3522,14 @@ static int vcycle_fixed(Lvl<double>* lv, int L, const wf_case& c, cudaStream_t s
   for (int l = 0; l < L; ++l) {
     if (l > 0) {
       // k_restrict also zeroes the coarse phi, ring included
-      WF_CK(launch_k(k_restrict<double>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s,
-          lv[l - 1], const_cast<double*>(lv[l].rhs), lv[l]));
+      WF_CK(launch_chain(k_restrict<double>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s,
+          lv[l - 1], const_cast<double*>(lv[l].rhs), lv[l], c.n_pre > 0 ? 1 : 0));
       WF_CKL("k_restrict");
     }
     WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, false, l > 0 && l == L - 1));
   }
   for (int l = L - 2; l >= 0; --l) {
-    WF_CK(launch_k(k_prolong<double>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s, 
+    WF_CK(launch_chain(k_prolong<double>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s, 
         lv[l + 1], lv[l]));
     WF_CKL("k_prolong");
     WF_TRY(relax(lv[l], c.n_post, s));
@@ -3603,7 +3634,7 @@ __device__ __forceinline__ double seam_coef(bool edge, int phys, int bit, double
 }
 
 __global__ void __launch_bounds__(MG_TPB) k_rk_rbgs(const Lvl<double> L, int phys, int color) {
-  pdl_entry();
+  pdl_chain();
   const int n = L.n;
   const int kx = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
   const int i = blockIdx.z;
@@ -3622,7 +3653,7 @@ __global__ void __launch_bounds__(MG_TPB) k_rk_rbgs(const Lvl<double> L, int phy
 }
 
 __global__ void k_rk_mirror(const Lvl<double> L, int phys) {
-  pdl_entry();
+  pdl_chain();
   const int n = L.n;
   const long tot = (long)n * n;
   for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < tot;
@@ -3640,7 +3671,7 @@ __global__ void k_rk_mirror(const Lvl<double> L, int phys) {
 
 __global__ void __launch_bounds__(MG_TPB) k_rk_restrict(const Lvl<double> F, Lvl<double> C,
                                                         int phys) {
-  pdl_entry();
+  pdl_chain();
   const int nc = C.n, n = F.n;
   const int ck = blockIdx.x * 32 + threadIdx.x, cj = blockIdx.y * 8 + threadIdx.y;
   const int ci = blockIdx.z;
@@ -3674,7 +3705,7 @@ __global__ void __launch_bounds__(MG_TPB) k_rk_restrict(const Lvl<double> F, Lvl
 }
 
 __global__ void __launch_bounds__(MG_TPB) k_rk_prolong(const Lvl<double> C, Lvl<double> F) {
-  pdl_entry();
+  pdl_chain();
   const int n = F.n;
   const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
   const int i = blockIdx.z;

@@ -26,7 +26,8 @@ namespace wf {
 static thread_local std::string g_err;
 thread_local long g_launches = 0;
 // Set while a stepper created with WF_STEP_SERIAL captures or launches: 1 no
-// programmatic dependent launch, 2 (WF_STEP_CHAIN) for the half-sweeps only.
+// programmatic dependent launch, 2 (WF_STEP_CHAIN) for the fills and the
+// multigrid only.
 static thread_local int g_pdl_off = 0;
 
 bool pdl_enabled(bool chain) {
@@ -56,7 +57,7 @@ struct BatchScope {
 };
 
 // Turns programmatic dependent launch off on this thread for one scope
-// (chain: except for the half-sweeps).
+// (chain: except for the fills and the multigrid).
 struct PdlOff {
   int prev;
   explicit PdlOff(bool on, bool chain = false) : prev(g_pdl_off) {
@@ -149,7 +150,7 @@ struct wf_stepper {
   wf_case c;
   int mode;     // 0 graph, 1 host loop
   int serial;   // WF_STEP_SERIAL: no programmatic dependent launch
-  int chain;    // WF_STEP_CHAIN: but for the half-sweeps
+  int chain;    // WF_STEP_CHAIN: but for the fills and the multigrid
   int32_t counts[4];  // launches: prologue, calmas pass, multigrid part, epilogue
   cudaGraph_t graph;
   cudaGraphExec_t exec;

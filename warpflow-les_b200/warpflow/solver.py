@@ -37,13 +37,13 @@ ALFARK = (0.5, 1.0)  # Heun RK2 stage coefficients (reference solver.py:26)
 
 STEP_MODES = {"graph": 0, "host": 1}
 STEP_SERIAL = 2   # WF_STEP_SERIAL: no programmatic dependent launch
-STEP_CHAIN = 8    # WF_STEP_CHAIN: but for the half-sweeps
+STEP_CHAIN = 8    # WF_STEP_CHAIN: but for the fills and the multigrid
 
 
 class FlowSolver:
     def __init__(self, cfg, topo, device, step_mode=None, serial=True):
         """`serial` (the default) builds the step without programmatic
-        dependent launch, but for the multigrid half-sweeps: every other
+        dependent launch, but for the fills and the multigrid: every other
         kernel's CTAs become resident only after the previous kernel
         finished, and solvers stepping concurrently find the SMs free.
         Measured on B200, us per step, none / half-sweeps / all kernels:
