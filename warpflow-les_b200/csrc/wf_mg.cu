@@ -439,7 +439,7 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0,
 // ring is not needed there because every ring term has a zero coefficient.
 // After the last sweep the interior and the face rings go back to global.
 template <class T>
-__global__ void __launch_bounds__(1024) k_relax_smem(Lvl<T> L0, int nsweeps, const Batch bt) {
+__global__ void __launch_bounds__(512) k_relax_smem(Lvl<T> L0, int nsweeps, const Batch bt) {
   pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
@@ -544,9 +544,19 @@ __device__ __forceinline__ void half_sweep_cols(const T* __restrict__ oth, T* __
 // division; correcting it to the exact quotient lengthens the dependent
 // chain of every update, which is what these latency-bound kernels cannot
 // afford).  Ring terms have zero coefficients and are not read.
+//
+// A relax of few sweeps is mostly its load and store, and a column per lane
+// would touch 32 rows with every access.  So the level moves row by row (lanes
+// along k) between global and shared memory, a plane's pitch odd so that the
+// cells of a row fall into different banks, and the columns come from there.
+// pre: the rhs is read ahead of the wait (complete before the launch ahead);
+// zero: phi is zero and not read.  6 sweeps of FP64, us:
+// 8^3 5.2 -> 3.7, 16^3 12.5 -> 8.5, 24^3 66.7 -> 27.6; a 32^3 step 410 -> 371.
 template <int NC>
 struct CoarseShape {
   static constexpr int THREADS = 2 * (((NC * (NC / 2)) + 31) / 32) * 32;
+  static constexpr int PLANE = NC * (NC / 2) + 1;              // one parity, one k plane
+  static constexpr int NIT = (NC * NC * NC + THREADS - 1) / THREADS;
 };
 
 // With unit_out set, CTA b relaxes rhs = e_u from phi = 0, u the b-th cell
@@ -555,21 +565,34 @@ struct CoarseShape {
 // index / 2): the rows of the coarse-level operator.
 template <class T, int NC, bool RHS_SMEM>
 __global__ void __launch_bounds__(CoarseShape<NC>::THREADS) k_coarse_cols(Lvl<T> L0,
-                                                                           int nsweeps,
-                                                                           T* unit_out,
+                                                                           int nsweeps, int pre,
+                                                                           int zero, T* unit_out,
                                                                            const int* unit_ids,
                                                                            const Batch bt) {
-  pdl_chain();
-  if (bt_skip(bt)) return;
+  if (bt.tab) {
+    pdl_chain();
+    if (bt_skip(bt)) return;
+    pre = 0;
+  }
   const Lvl<T> L = rebase(L0, bt);
   constexpr int H = NC / 2;
   constexpr int HALF = NC * H;                  // columns per parity
   constexpr int GROUP = ((HALF + 31) / 32) * 32;
-  constexpr int PLANE = NC * H;                 // one parity, one k plane
+  constexpr int THREADS = CoarseShape<NC>::THREADS, NIT = CoarseShape<NC>::NIT;
+  constexpr int PLANE = CoarseShape<NC>::PLANE;
   extern __shared__ __align__(16) unsigned char smraw[];
   T* sp = reinterpret_cast<T*>(smraw);
-  T* srh = sp + NC * NC * NC;                   // rhs, when it stays in smem
+  T* srh = sp + 2 * NC * PLANE;                 // rhs, laid out as phi
   const int tid = threadIdx.x;
+  T rv[NIT];
+  if (pre && !unit_out) {
+#pragma unroll
+    for (int q = 0; q < NIT; ++q) {
+      const int t = tid + q * THREADS;
+      if (t < NC * NC * NC)
+        rv[q] = __ldcg(L.rhs + lid(L, t / (NC * NC) + 1, t / NC % NC + 1, t % NC + 1));
+    }
+  }
   const int g = tid / GROUP;                    // 0: (i+j) even, 1: odd
   const int q = tid - g * GROUP;
   const bool active = q < HALF;
@@ -592,27 +615,52 @@ __global__ void __launch_bounds__(CoarseShape<NC>::THREADS) k_coarse_cols(Lvl<T>
   const T inv_hi = T(1) / (-(aw + ae + as + an + az + T(0)));
   T ph[NC];
   T rh[RHS_SMEM ? 1 : NC];
-  const long c0 = lid(L, i + 1, j + 1, 1);
   // the unit cell of this CTA: the one of cells 2b, 2b+1 with even i+j+k,
   // b = unit_ids[blockIdx.x] (or blockIdx.x)
   const int ub = unit_ids ? unit_ids[blockIdx.x] : (int)blockIdx.x;
   const int unit = 2 * ub + (((2 * ub / NC) / NC + (2 * ub / NC) % NC) & 1);
+  if (!bt.tab) pdl_chain();
+  if (unit_out) {
 #pragma unroll
-  for (int k = 0; k < NC; ++k) {
-    T r;
-    if (unit_out) {
+    for (int k = 0; k < NC; ++k) {
       ph[k] = T(0);
-      r = (active && (i * NC + j) * NC + k == unit) ? T(1) : T(0);
-    } else {
-      ph[k] = active ? L.phi[c0 + k] : T(0);
-      r = active ? L.rhs[c0 + k] : T(0);
+      const T r = (active && (i * NC + j) * NC + k == unit) ? T(1) : T(0);
+      if (!RHS_SMEM) rh[RHS_SMEM ? 0 : k] = r;
+      else if (active) srh[(g * NC + k) * PLANE + me] = r;
+      if (active) own[k * PLANE + me] = T(0);
     }
-    if (RHS_SMEM) {
-      if (active) srh[(g * NC + k) * PLANE + me] = r;
-    } else {
-      rh[RHS_SMEM ? 0 : k] = r;
+  } else {
+    // one array after the other (registers); in a V-cycle the rhs came ahead
+    // of the wait or phi is zero
+    auto at = [&](int t) {
+      const int a = t / (NC * NC), b = t / NC % NC, d = t % NC;
+      return (((a + b) & 1) * NC + d) * PLANE + a * H + (b >> 1);
+    };
+    auto load = [&](const T* src) {
+#pragma unroll
+      for (int q = 0; q < NIT; ++q) {
+        const int t = tid + q * THREADS;
+        if (t < NC * NC * NC)
+          rv[q] = src[lid(L, t / (NC * NC) + 1, t / NC % NC + 1, t % NC + 1)];
+      }
+    };
+    auto stage = [&](T* dst) {
+#pragma unroll
+      for (int q = 0; q < NIT; ++q) {
+        const int t = tid + q * THREADS;
+        if (t < NC * NC * NC) dst[at(t)] = zero && dst == sp ? T(0) : rv[q];
+      }
+    };
+    if (!pre) load(L.rhs);
+    stage(srh);
+    if (!zero) load(L.phi);
+    stage(sp);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+      ph[k] = own[k * PLANE + me];
+      if (!RHS_SMEM) rh[RHS_SMEM ? 0 : k] = srh[(g * NC + k) * PLANE + me];
     }
-    if (active) own[k * PLANE + me] = ph[k];
   }
   __syncthreads();
   for (int sw = 0; sw < nsweeps; ++sw) {
@@ -631,47 +679,53 @@ __global__ void __launch_bounds__(CoarseShape<NC>::THREADS) k_coarse_cols(Lvl<T>
       __syncthreads();
     }
   }
-  if (!active) return;
   if (unit_out) {
+    if (!active) return;
     T* row = unit_out + (long)blockIdx.x * (NC * NC * NC / 2) + ((i * NC + j) * NC >> 1);
 #pragma unroll
     for (int k = 0; k < NC; ++k)
       if (((i + j + k) & 1) == 0) row[k >> 1] = ph[k];
     return;
   }
+  // the last half-sweep's barrier has published every column
 #pragma unroll
-  for (int k = 0; k < NC; ++k) {
-    const long c = c0 + k;
-    L.phi[c] = ph[k];
-    if (nsweeps > 0) ring_mirror(L, i, j, k, c, ph[k]);
+  for (int q = 0; q < NIT; ++q) {
+    const int t = tid + q * THREADS;
+    if (t < NC * NC * NC) {
+      const int a = t / (NC * NC), b = t / NC % NC, d = t % NC;
+      const T x = sp[(((a + b) & 1) * NC + d) * PLANE + a * H + (b >> 1)];
+      const long c = lid(L, a + 1, b + 1, d + 1);
+      L.phi[c] = x;
+      if (nsweeps > 0) ring_mirror(L, a, b, d, c, x);
+    }
   }
 }
 
 template <class T, int NC, bool RHS_SMEM>
-static int launch_coarse(const Lvl<T>& L, int nsweeps, cudaStream_t s, T* unit_out = nullptr,
-                         const int* unit_ids = nullptr, int nunits = 0) {
-  constexpr int HALF = NC * (NC / 2);
-  constexpr int GROUP = ((HALF + 31) / 32) * 32;
-  const size_t sb = (size_t)NC * NC * NC * sizeof(T) * (RHS_SMEM ? 2 : 1);
+static int launch_coarse(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool pre, bool zero,
+                         T* unit_out = nullptr, const int* unit_ids = nullptr, int nunits = 0) {
+  const size_t lvl = (size_t)2 * NC * CoarseShape<NC>::PLANE * sizeof(T);
+  const size_t sb = RHS_SMEM || !unit_out ? 2 * lvl : lvl;
   WF_CK(cudaFuncSetAttribute(k_coarse_cols<T, NC, RHS_SMEM>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb));
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * lvl)));
   const int nb = unit_out ? (unit_ids ? nunits : NC * NC * NC / 2) : 1;
-  WF_CK(launch_k(k_coarse_cols<T, NC, RHS_SMEM>, nb, 2 * GROUP, sb, s, L, nsweeps, unit_out,
-                 unit_ids));
+  WF_CK(launch_chain(k_coarse_cols<T, NC, RHS_SMEM>, nb, CoarseShape<NC>::THREADS, sb, s, L,
+                     nsweeps, pre ? 1 : 0, zero ? 1 : 0, unit_out, unit_ids));
   WF_CKL("k_coarse_cols");
   return WF_OK;
 }
 
 // returns 1 when a specialised coarse kernel handled the level
 template <class T>
-static int try_coarse(const Lvl<T>& L, int nsweeps, cudaStream_t s, int* rc) {
+static int try_coarse(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool pre, bool zero,
+                      int* rc) {
   switch (L.n) {
-    case 4: *rc = launch_coarse<T, 4, false>(L, nsweeps, s); return 1;
-    case 8: *rc = launch_coarse<T, 8, false>(L, nsweeps, s); return 1;
-    case 12: *rc = launch_coarse<T, 12, false>(L, nsweeps, s); return 1;
-    case 16: *rc = launch_coarse<T, 16, false>(L, nsweeps, s); return 1;
-    case 20: *rc = launch_coarse<T, 20, false>(L, nsweeps, s); return 1;
-    case 24: *rc = launch_coarse<T, 24, true>(L, nsweeps, s); return 1;
+    case 4: *rc = launch_coarse<T, 4, false>(L, nsweeps, s, pre, zero); return 1;
+    case 8: *rc = launch_coarse<T, 8, false>(L, nsweeps, s, pre, zero); return 1;
+    case 12: *rc = launch_coarse<T, 12, false>(L, nsweeps, s, pre, zero); return 1;
+    case 16: *rc = launch_coarse<T, 16, false>(L, nsweeps, s, pre, zero); return 1;
+    case 20: *rc = launch_coarse<T, 20, false>(L, nsweeps, s, pre, zero); return 1;
+    case 24: *rc = launch_coarse<T, 24, true>(L, nsweeps, s, pre, zero); return 1;
     default: return 0;
   }
 }
@@ -2045,12 +2099,12 @@ static int build_coarse_op(const Lvl<T>& L, int n_coarse, T* op, cudaStream_t s)
   // process), so it may stay asynchronous
   const int nsweeps = n_coarse - 1;
   switch (L.n) {
-    case 4: return launch_coarse<T, 4, false>(L, nsweeps, s, op, ints, P.nrep);
-    case 8: return launch_coarse<T, 8, false>(L, nsweeps, s, op, ints, P.nrep);
-    case 12: return launch_coarse<T, 12, false>(L, nsweeps, s, op, ints, P.nrep);
-    case 16: return launch_coarse<T, 16, false>(L, nsweeps, s, op, ints, P.nrep);
-    case 20: return launch_coarse<T, 20, false>(L, nsweeps, s, op, ints, P.nrep);
-    default: return launch_coarse<T, 24, true>(L, nsweeps, s, op, ints, P.nrep);
+    case 4: return launch_coarse<T, 4, false>(L, nsweeps, s, false, true, op, ints, P.nrep);
+    case 8: return launch_coarse<T, 8, false>(L, nsweeps, s, false, true, op, ints, P.nrep);
+    case 12: return launch_coarse<T, 12, false>(L, nsweeps, s, false, true, op, ints, P.nrep);
+    case 16: return launch_coarse<T, 16, false>(L, nsweeps, s, false, true, op, ints, P.nrep);
+    case 20: return launch_coarse<T, 20, false>(L, nsweeps, s, false, true, op, ints, P.nrep);
+    default: return launch_coarse<T, 24, true>(L, nsweeps, s, false, true, op, ints, P.nrep);
   }
 }
 
@@ -2917,23 +2971,17 @@ static inline int mg_blocks(long work) {
   return (int)std::max<long>(b, 1);
 }
 
-template <class T>
-static size_t smem_bytes(int n) {
-  return 2ull * (size_t)n * n * n * sizeof(T);
-}
-
-constexpr size_t SMEM_CAP = 220 * 1024;
-
 // rhs_ready: the level's rhs is unchanged since its last relax, so a split
 // copy of it made then can be reused
-// zero: the level's phi is zero (a coarsest level after the restriction)
+// zero: the level's phi is zero (a level after the restriction)
+// last: the coarsest level
 template <class T>
 static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = false,
-                 bool zero = false) {
+                 bool zero = false, bool last = false) {
   if (nsweeps <= 0) return WF_OK;
   {
     int rc = WF_OK;
-    if (zero && try_coarse_cheb(L, nsweeps, s, &rc)) return rc;
+    if (zero && last && try_coarse_cheb(L, nsweeps, s, &rc)) return rc;
   }
   // a bucket launch serves many cases through their table: only kernels that
   // take one (the one-CTA column kernel, split and plain sweeps, the
@@ -2948,7 +2996,12 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
     if (nsweeps > 12 && strat == 3 && try_coarse_tb<T>(L, nsweeps, s, &rc)) return rc;
     if (nsweeps > 12 && strat == 2 && try_coarse_p2p<T>(L, nsweeps, s, &rc)) return rc;
     if (nsweeps > 12 && strat == 1 && try_coarse_cluster<T>(L, nsweeps, s, &rc)) return rc;
-    if (try_coarse<T>(L, nsweeps, s, &rc)) return rc;
+    // FP64 from 20 with few sweeps: a launch per half-sweep.  6 sweeps of
+    // 20^3 / 24^3: one CTA 20.3 / 27.5 us, launches 13.7 / 14.0 (16^3: 8.5 and
+    // 13.5).  Not FP32, whose last bit the quotient in place of the reciprocal
+    // would change.
+    const bool launches = sizeof(T) == 8 && L.n >= 20 && nsweeps <= 12;
+    if (!launches && try_coarse<T>(L, nsweeps, s, rhs_ready, zero, &rc)) return rc;
     if (!bucket && nsweeps > 12 && try_coarse_exact<T>(L, nsweeps, s, &rc)) return rc;
   }
   if (L.tmp && (L.n & 1) == 0 && L.n >= split_min_n())
@@ -2976,14 +3029,13 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
     WF_TRY(launch_relax_persist<T>(L, nsweeps, s, &done));
     if (done) return WF_OK;
   }
-  const size_t sb = smem_bytes<T>(L.n);
-  if (sb <= SMEM_CAP) {
-    WF_CK(cudaFuncSetAttribute(k_relax_smem<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)SMEM_CAP));
+  // up to 10 one CTA sweeps in shared memory, from 11 each half-sweep is a
+  // launch (the same bits).  us for 6 sweeps, one CTA / launches: 10^3 11.5 /
+  // 15.1, 11^3 18.1 / 15.1, 14^3 25.2 / 13.6, 18^3 45.0 / 13.7, 22^3 78.0 / 14.0
+  if (L.n <= 10) {
     const int n3 = L.n * L.n * L.n;
-    int tpb = 1024;
-    if (n3 / 2 < 1024) tpb = std::max(32, ((n3 / 2 + 31) / 32) * 32);
-    WF_CK(launch_k(k_relax_smem<T>, 1, tpb, sb, s, L, nsweeps));
+    const int tpb = (n3 / 2 + 31) / 32 * 32;
+    WF_CK(launch_chain(k_relax_smem<T>, 1, std::max(32, tpb), 2 * n3 * sizeof(T), s, L, nsweeps));
     WF_CKL("k_relax_smem");
     return WF_OK;
   }
@@ -3035,7 +3087,7 @@ static int vcycle(std::vector<Lvl<T>>& lv, const wf_case& c, cudaStream_t s,
       WF_TRY(split_sweeps(lv[l], c.n_pre, s));
     else
       WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, l == 0 && rhs0_ready,
-                   l > 0 && l == L - 1));
+                   l > 0, l == L - 1));
   }
   for (int l = L - 2; l >= 0; --l) {
     // fine levels from 64: one thread per coarse cell (fewer loads); smaller
@@ -3526,7 +3578,7 @@ static int vcycle_fixed(Lvl<double>* lv, int L, const wf_case& c, cudaStream_t s
           lv[l - 1], const_cast<double*>(lv[l].rhs), lv[l], c.n_pre > 0 ? 1 : 0));
       WF_CKL("k_restrict");
     }
-    WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, false, l > 0 && l == L - 1));
+    WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, false, l > 0, l == L - 1));
   }
   for (int l = L - 2; l >= 0; --l) {
     WF_CK(launch_chain(k_prolong<double>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s, 
