@@ -198,8 +198,45 @@ static int launch_rbgs(const Lvl<T>& L, int color, bool pre, cudaStream_t s) {
   return WF_OK;
 }
 
+// The first half-sweep of a level whose phi is zero: colour 0 becomes rhs/ap,
+// the other colour stays zero, and it needs nothing but the rhs.  So the kernel
+// that writes such a level's rhs (restriction, defect, the copy into the split
+// layout) writes this in place of the zeros, and the half-sweep's launch and
+// its pass over memory are gone; the quotient is exact, so the bits are the
+// half-sweep's.  Left in the cell, its face-ring mirrors, and zero in the other
+// ring cells nearest to it, so that the real cells' threads together write
+// every cell of the (n+2)^3 array exactly once.  first 0: zeros.
+//   FIRST_FIGURES
+template <class T>
+__device__ __forceinline__ T first_value(const Lvl<T>& L, const ApRecip<T>& rt, int i, int j, int k,
+                                         T r) {
+  const int n = L.n;
+  if (((i + j + k) & 1) == 0) return T(0);
+  const T aw = i > 0 ? L.ax : T(0), ae = i < n - 1 ? L.ax : T(0);
+  const T as = j > 0 ? L.ay : T(0), an = j < n - 1 ? L.ay : T(0);
+  const T ab = k > 0 ? L.az : T(0), at = k < n - 1 ? L.az : T(0);
+  return div_by_recip(r, -(aw + ae + as + an + ab + at),
+                      rt.y[9 * ((i > 0) + (i < n - 1)) + 3 * ((j > 0) + (j < n - 1)) + (k > 0) +
+                           (k < n - 1)]);
+}
+
+template <class T>
+__device__ __forceinline__ void start_cell(const Lvl<T>& L, const ApRecip<T>& rt, int first, int i,
+                                           int j, int k, T r) {
+  const int n = L.n;
+  const T x = first ? first_value(L, rt, i, j, k, r) : T(0);
+  const int zi0 = i == 0 ? -1 : 0, zi1 = i == n - 1 ? 1 : 0;
+  const int zj0 = j == 0 ? -1 : 0, zj1 = j == n - 1 ? 1 : 0;
+  const int zk0 = k == 0 ? -1 : 0, zk1 = k == n - 1 ? 1 : 0;
+  for (int oi = zi0; oi <= zi1; ++oi)
+    for (int oj = zj0; oj <= zj1; ++oj)
+      for (int ok = zk0; ok <= zk1; ++ok)
+        L.phi[lid(L, i + 1 + oi, j + 1 + oj, k + 1 + ok)] =
+            (oi != 0) + (oj != 0) + (ok != 0) <= 1 ? x : T(0);
+}
+
 // restriction (multigrid.py:93-119): rhs_c = 1/8 sum of the 8 fine residuals;
-// also zeroes the coarse level's phi, ring included.  A short launch at coarse
+// also starts the coarse level's phi (start_cell), ring included.  A short launch at coarse
 // sizes: the indices and, with pre, the eight fine rhs values come ahead of the
 // wait.  This, the same in the prolongations (fine phi) and the coarse-operator
 // kernels, all in the chain, with k_cop_gemm's four representatives to a warp:
@@ -207,7 +244,9 @@ static int launch_rbgs(const Lvl<T>& L, int color, bool pre, cudaStream_t s) {
 // 1520 -> 1500, 256^3 FP64 unchanged (its transfers are bandwidth)
 template <class T>
 __global__ void __launch_bounds__(MG_TPB) k_restrict(const Lvl<T> F0, T* rhs_c, Lvl<T> C0,
-                                                     int pre, const Batch bt) {
+                                                     int pre, int first,
+                                                     const __grid_constant__ ApRecip<T> rt,
+                                                     const Batch bt) {
   if (bt.tab) {
     pdl_chain();
     if (bt_skip(bt)) return;
@@ -271,17 +310,10 @@ __global__ void __launch_bounds__(MG_TPB) k_restrict(const Lvl<T> F0, T* rhs_c, 
                              ap * P[a][b][q]);
           acc = acc + res;
         }
-    rhs_c[lid(C, ci + 1, cj + 1, ck + 1)] = acc * T(0.125);
-    // the coarse phi starts from zero (multigrid.py:314): this cell and the
-    // ring cells nearest to it (faces, edges, corners), so that every cell
-    // of the (nc+2)^3 array is zeroed exactly once
-    const int zi0 = ci == 0 ? -1 : 0, zi1 = ci == nc - 1 ? 1 : 0;
-    const int zj0 = cj == 0 ? -1 : 0, zj1 = cj == nc - 1 ? 1 : 0;
-    const int zk0 = ck == 0 ? -1 : 0, zk1 = ck == nc - 1 ? 1 : 0;
-    for (int oi = zi0; oi <= zi1; ++oi)
-      for (int oj = zj0; oj <= zj1; ++oj)
-        for (int ok = zk0; ok <= zk1; ++ok)
-          C.phi[lid(C, ci + 1 + oi, cj + 1 + oj, ck + 1 + ok)] = T(0);
+    const T v = acc * T(0.125);
+    rhs_c[lid(C, ci + 1, cj + 1, ck + 1)] = v;
+    // the coarse phi starts from zero (multigrid.py:314)
+    start_cell(C, rt, first, ci, cj, ck, v);
   }
 }
 
@@ -310,9 +342,11 @@ __global__ void k_zero_strided(T* a, int m, long sI, long sJ) {
   }
 }
 
-// prolongation (multigrid.py:122-146) + the ring refill that follows it
+// prolongation (multigrid.py:122-146) + the ring refill that follows it; half:
+// only into the cells the next half-sweep (colour 0) does not overwrite
 template <class T>
-__global__ void __launch_bounds__(MG_TPB) k_prolong(const Lvl<T> C0, Lvl<T> F0, const Batch bt) {
+__global__ void __launch_bounds__(MG_TPB) k_prolong(const Lvl<T> C0, Lvl<T> F0, int half,
+                                                    const Batch bt) {
   if (bt.tab) {
     pdl_chain();
     if (bt_skip(bt)) return;
@@ -320,10 +354,12 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong(const Lvl<T> C0, Lvl<T> F0, 
   const Lvl<T> C = rebase(C0, bt);
   const Lvl<T> F = rebase(F0, bt);
   const int n = F.n;
-  {  // one thread per cell: x = k (runs of 32), y = j (groups of 8), z = i
-    const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
-    const bool on = k < n && j < n;
+  {  // one thread per cell: x = k (runs of 32), y = j (groups of 8), z = i;
+     // half: x = the cells of a row with even i+j+k
+    const int x0 = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
     const int i = bt_z(bt);
+    const int k = half ? 2 * x0 + ((i + j) & 1) : x0;
+    const bool on = k < n && j < n;
     const long c = lid(F, i + 1, j + 1, k + 1);
     // written before the restriction out of this level (pdl_chain)
     const T old = on ? __ldcg(F.phi + c) : T(0);
@@ -355,6 +391,8 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong(const Lvl<T> C0, Lvl<T> F0, 
   }
 }
 
+static dim3 prolong_grid(int n, int half) { return cells3(n, n, half ? (n + 1) / 2 : n); }
+
 // the same prolongation with one thread per COARSE cell writing its 2x2x2
 // fine cells from the 27 coarse values around it, each loaded once (27 loads
 // for 8 outputs instead of 64); every output sums the same terms in the
@@ -365,7 +403,8 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong(const Lvl<T> C0, Lvl<T> F0, 
 // Loading them first is safe because each fine cell is written by this
 // thread only, and ring_mirror writes ring cells, which are never loaded.
 template <class T>
-__global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0, const Batch bt) {
+__global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0, int half,
+                                                     const Batch bt) {
   if (bt.tab) {
     pdl_chain();
     if (bt_skip(bt)) return;
@@ -387,7 +426,8 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0,
 #pragma unroll
       for (int pk = 0; pk < 2; ++pk) {
         fc[pi][pj][pk] = lid(F, 2 * ci + pi + 1, 2 * cj + pj + 1, 2 * ck + pk + 1);
-        fv[pi][pj][pk] = on ? __ldcg(F.phi + fc[pi][pj][pk]) : T(0);
+        fv[pi][pj][pk] =
+            on && !(half && ((pi + pj + pk) & 1)) ? __ldcg(F.phi + fc[pi][pj][pk]) : T(0);
       }
   if (!bt.tab) pdl_chain();
   if (!on) return;
@@ -409,6 +449,7 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0,
     for (int pj = 0; pj < 2; ++pj)
 #pragma unroll
       for (int pk = 0; pk < 2; ++pk) {
+        if (half && ((pi + pj + pk) & 1)) continue;
         const T wx0 = pi == 0 ? T(0.25) : T(0.75);
         const T wy0 = pj == 0 ? T(0.25) : T(0.75);
         const T wz0 = pk == 0 ? T(0.25) : T(0.75);
@@ -2175,10 +2216,12 @@ static int try_coarse_cluster(const Lvl<T>& L, int nsweeps, cudaStream_t s, int*
 // mirrors, which is what k_rbgs leaves in the ring after the last sweep.
 constexpr int SPLIT_ROWS = 8;  // rows (one warp each) per CTA
 
-// level phi (all (n+2)^3 cells) and rhs -> split copies sp, sr (dense strides)
+// level phi (all (n+2)^3 cells) and rhs -> split copies sp, sr (dense strides);
+// first (with_rhs set): phi is zero and is not read, first_value takes its place
 template <class T>
 __global__ void __launch_bounds__(32 * SPLIT_ROWS)
-    k_split_in(const Lvl<T> L0, T* sp, T* sr, int with_rhs, const Batch bt) {
+    k_split_in(const Lvl<T> L0, T* sp, T* sr, int with_rhs, int first,
+               const __grid_constant__ ApRecip<T> rt, const Batch bt) {
   pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
@@ -2194,8 +2237,10 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
   const long dst = (long)i * L.tI + (long)j * L.tJ;
   for (int a = threadIdx.x & 31; a < m; a += 32) {
     const int q = spos(a, H);
-    const T x = L.phi[src + a];
+    T x = first ? T(0) : L.phi[src + a];
     const T y = with_rhs ? L.rhs[src + a] : T(0);   // both loads before the stores
+    if (first && i > 0 && i < m - 1 && j > 0 && j < m - 1 && a > 0 && a < m - 1)
+      x = first_value(L, rt, i - 1, j - 1, a - 1, y);
     sp[dst + q] = x;
     if (with_rhs) sr[dst + q] = y;
   }
@@ -2463,12 +2508,12 @@ static int split_min_n() {
 
 // level -> split copies (phi, and rhs unless the scratch already holds it)
 template <class T>
-static int split_in(const Lvl<T>& L, bool with_rhs, cudaStream_t s) {
+static int split_in(const Lvl<T>& L, bool with_rhs, cudaStream_t s, bool first = false) {
   const int m = L.n + 2;
   T* sp = split_phi(L.tmp);
   T* sr = split_rhs(L.tmp, L.n);
   WF_CK(launch_k(k_split_in<T>, (m * m + SPLIT_ROWS - 1) / SPLIT_ROWS, 32 * SPLIT_ROWS, 0, s, L,
-                 sp, sr, with_rhs ? 1 : 0));
+                 sp, sr, with_rhs || first ? 1 : 0, first ? 1 : 0, ap_recip(L)));
   WF_CKL("k_split_in");
   return WF_OK;
 }
@@ -2490,9 +2535,11 @@ static int split_in(const Lvl<T>& L, bool with_rhs, cudaStream_t s) {
 //    (what the one before touched last is still in L2: 256^3 FP64 41.5 -> 40.0).
 //  - Otherwise, and for a shape set for the level (wf_set_launch_shape), the
 //    rows of k_rbgs_split.
-// rhs_ready: the split rhs was complete before the launch ahead of the first one
+// rhs_ready: the split rhs was complete before the launch ahead of the first one;
+// first: the launch ahead made the first half-sweep (first_value)
 template <class T>
-static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = false) {
+static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = false,
+                        bool first = false) {
   const int n = L.n, nh = n / 2;
   T* sp = split_phi(L.tmp);
   const T* sr = split_rhs(L.tmp, n);
@@ -2513,9 +2560,9 @@ static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_r
               : cpt == 2 ? k_rbgs_split<T, 2>
                          : k_rbgs_split<T, 1>;
   auto kflat = cells == 2 ? k_rbgs_flat<T, 2> : k_rbgs_flat<T, 1>;
-  for (int h = 0; h < 2 * nsweeps; ++h) {
-    // from the second half-sweep on, the launch ahead is a half-sweep
-    const int pre = h > 0 || rhs_ready ? 1 : 0, color = h & 1, back = n >= 176 ? color : 0;
+  for (int h = first ? 1 : 0; h < 2 * nsweeps; ++h) {
+    // after the first of these launches, the launch ahead is a half-sweep
+    const int pre = h > (first ? 1 : 0) || rhs_ready ? 1 : 0, color = h & 1, back = n >= 176 ? color : 0;
     if (flat)
       WF_CK(launch_chain(kflat, fgrid, MG_TPB, 0, s, L, sp, sr, color, pre, 1.0f / (float)nh, rt));
     else if (pair)
@@ -2971,14 +3018,39 @@ static inline int mg_blocks(long work) {
   return (int)std::max<long>(b, 1);
 }
 
+// a level of the V-cycle whose relax is a plain launch per half-sweep
+template <class T>
+static bool relax_by_launches(const Lvl<T>& L, int nsweeps) {
+  if (nsweeps < 1 || nsweeps > 12 || L.n < 11) return false;
+  // one CTA (k_coarse_cols) up to 24.  FP64 from 20 takes launches: 6 sweeps of
+  // 20^3 / 24^3 in one CTA 20.3 / 27.5 us, by launches 13.7 / 14.0 (16^3: 8.5 and
+  // 13.5).  Not FP32, whose last bit the quotient in place of the reciprocal
+  // would change.
+  if (L.n <= 24 && L.n % 4 == 0 && !(sizeof(T) == 8 && L.n >= 20)) return false;
+  if (L.tmp && (L.n & 1) == 0 && L.n >= split_min_n()) return false;
+  return batch_ctx().tab || !(mid_p2p_enabled() || (L.tmp && L.n >= sweep2_min_n()) ||
+                              (L.gbar && L.n >= persist_min_n()));
+}
+
+// the half-sweeps of such a relax; first: the launch ahead made the first one
+template <class T>
+static int launch_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready,
+                         bool first) {
+  for (int h = first ? 1 : 0; h < 2 * nsweeps; ++h)
+    WF_TRY(launch_rbgs(L, h & 1, h > (first ? 1 : 0) || rhs_ready, s));
+  return WF_OK;
+}
+
 // rhs_ready: the level's rhs is unchanged since its last relax, so a split
 // copy of it made then can be reused
 // zero: the level's phi is zero (a level after the restriction)
-// last: the coarsest level
+// last: the coarsest level; first: the launch ahead made the first half-sweep
+// (only where relax_by_launches)
 template <class T>
 static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = false,
-                 bool zero = false, bool last = false) {
+                 bool zero = false, bool last = false, bool first = false) {
   if (nsweeps <= 0) return WF_OK;
+  if (relax_by_launches(L, nsweeps)) return launch_sweeps(L, nsweeps, s, rhs_ready, first);
   {
     int rc = WF_OK;
     if (zero && last && try_coarse_cheb(L, nsweeps, s, &rc)) return rc;
@@ -2996,12 +3068,7 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
     if (nsweeps > 12 && strat == 3 && try_coarse_tb<T>(L, nsweeps, s, &rc)) return rc;
     if (nsweeps > 12 && strat == 2 && try_coarse_p2p<T>(L, nsweeps, s, &rc)) return rc;
     if (nsweeps > 12 && strat == 1 && try_coarse_cluster<T>(L, nsweeps, s, &rc)) return rc;
-    // FP64 from 20 with few sweeps: a launch per half-sweep.  6 sweeps of
-    // 20^3 / 24^3: one CTA 20.3 / 27.5 us, launches 13.7 / 14.0 (16^3: 8.5 and
-    // 13.5).  Not FP32, whose last bit the quotient in place of the reciprocal
-    // would change.
-    const bool launches = sizeof(T) == 8 && L.n >= 20 && nsweeps <= 12;
-    if (!launches && try_coarse<T>(L, nsweeps, s, rhs_ready, zero, &rc)) return rc;
+    if (try_coarse<T>(L, nsweeps, s, rhs_ready, zero, &rc)) return rc;
     if (!bucket && nsweeps > 12 && try_coarse_exact<T>(L, nsweeps, s, &rc)) return rc;
   }
   if (L.tmp && (L.n & 1) == 0 && L.n >= split_min_n())
@@ -3039,11 +3106,7 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
     WF_CKL("k_relax_smem");
     return WF_OK;
   }
-  for (int sw = 0; sw < nsweeps; ++sw) {
-    WF_TRY(launch_rbgs(L, 0, sw > 0 || rhs_ready, s));
-    WF_TRY(launch_rbgs(L, 1, true, s));
-  }
-  return WF_OK;
+  return launch_sweeps(L, nsweeps, s, rhs_ready, false);
 }
 
 // a level the V-cycle keeps in the split layout: one that relax() would send
@@ -3058,10 +3121,13 @@ static bool split_resident(const Lvl<T>& L, const wf_case& c) {
 // it (a solve's V-cycles share rhs = su).  split0_in: level 0's split copy
 // already holds its current phi (left there by the previous V-cycle);
 // split0_keep: leave the result in the split copy (the next V-cycle of the
-// same solve continues from it) instead of copying it back.
+// same solve continues from it) instead of copying it back.  first0: the
+// caller has already made level 0's first half-sweep (mixed precision);
+// zero0: level 0's phi is zero.
 template <class T>
 static int vcycle(std::vector<Lvl<T>>& lv, const wf_case& c, cudaStream_t s,
-                  bool rhs0_ready = false, bool split0_in = false, bool split0_keep = false) {
+                  bool rhs0_ready = false, bool split0_in = false, bool split0_keep = false,
+                  bool first0 = false, bool zero0 = false) {
   const int L = (int)lv.size();
   std::vector<Lvl<T>> vw(lv);    // the views restriction and prolongation work on
   std::vector<char> res(L, 0);   // level kept split from pre- to post-smoothing
@@ -3071,34 +3137,41 @@ static int vcycle(std::vector<Lvl<T>>& lv, const wf_case& c, cudaStream_t s,
       vw[l] = split_view(lv[l]);
     }
   for (int l = 0; l < L; ++l) {
+    bool first = l == 0 && first0;
     if (l > 0) {
       Lvl<T>& C = vw[l];
+      first = res[l] || (l < L - 1 && relax_by_launches(lv[l], c.n_pre));
       // the finer level's sweeps lie between its rhs and this launch
       WF_CK(launch_chain(k_restrict<T>, cells3(C.n, C.n, C.n), cell_block(), 0, s, vw[l - 1],
-                         const_cast<T*>(C.rhs), C, c.n_pre > 0 ? 1 : 0));
+                         const_cast<T*>(C.rhs), C, c.n_pre > 0 ? 1 : 0, first ? 1 : 0,
+                         ap_recip(C)));
       WF_CKL("k_restrict");
     } else if (res[0] && !split0_in) {
-      WF_TRY(split_in(lv[0], !rhs0_ready, s));
+      first = zero0;
+      WF_TRY(split_in(lv[0], !rhs0_ready, s, zero0));
     }
     if (l == L - 1 && L > 1 && c.mg_cop && c.mg_cop_part && c.n_coarse >= 2 &&
         cop_size_ok(lv[l].n))
       WF_TRY(apply_coarse_op<T>(lv[l], (const T*)c.mg_cop, (T*)c.mg_cop_part, s));
     else if (res[l])
-      WF_TRY(split_sweeps(lv[l], c.n_pre, s));
+      WF_TRY(split_sweeps(lv[l], c.n_pre, s, false, first));
     else
       WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, l == 0 && rhs0_ready,
-                   l > 0, l == L - 1));
+                   l > 0, l == L - 1, first));
   }
+  // the post-smoothing starts with colour 0, from the other colour alone: the
+  // prolongation need not make the cells it overwrites
+  const int half = c.n_post > 0 ? 1 : 0;
   for (int l = L - 2; l >= 0; --l) {
     // fine levels from 64: one thread per coarse cell (fewer loads); smaller
     // ones keep one thread per fine cell (more threads in flight)
     if (lv[l].n >= 64 && (lv[l].n & 1) == 0) {
       WF_CK(launch_chain(k_prolong8<T>, cells3(lv[l + 1].n, lv[l + 1].n, lv[l + 1].n), cell_block(),
-                     0, s, vw[l + 1], vw[l]));
+                     0, s, vw[l + 1], vw[l], half));
       WF_CKL("k_prolong8");
     } else {
-      WF_CK(launch_chain(k_prolong<T>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s,
-                     vw[l + 1], vw[l]));
+      WF_CK(launch_chain(k_prolong<T>, prolong_grid(lv[l].n, half), cell_block(), 0, s, vw[l + 1],
+                         vw[l], half));
       WF_CKL("k_prolong");
     }
     if (res[l]) {
@@ -3177,20 +3250,10 @@ __device__ __forceinline__ double defect_at(const Lvl<double>& F, int n, int i, 
                      an * p[c + F.sJ] + ab * p[c - 1] + at * p[c + 1] + ap * p[c]);
 }
 
-// zero cell (i, j, k) (0-based real index) of an FP32 level array and the
-// ring cells nearest to it (faces, edges, corners), so that the real cells'
-// threads together zero every cell of the (n+2)^3 array exactly once
-__device__ __forceinline__ void zero_with_ring(const Lvl<float>& L, int n, int i, int j, int k) {
-  const int zi0 = i == 0 ? -1 : 0, zi1 = i == n - 1 ? 1 : 0;
-  const int zj0 = j == 0 ? -1 : 0, zj1 = j == n - 1 ? 1 : 0;
-  const int zk0 = k == 0 ? -1 : 0, zk1 = k == n - 1 ? 1 : 0;
-  for (int oi = zi0; oi <= zi1; ++oi)
-    for (int oj = zj0; oj <= zj1; ++oj)
-      for (int ok = zk0; ok <= zk1; ++ok) L.phi[lid(L, i + 1 + oi, j + 1 + oj, k + 1 + ok)] = 0.0f;
-}
-
 // Lf: the FP32 level 0 (its own arrays, or with LV_SPLIT its split copies)
 __global__ void __launch_bounds__(MG_TPB) k_defect(const Lvl<double> F0, const Lvl<float> Lf0,
+                                                   int first,
+                                                   const __grid_constant__ ApRecip<float> rt,
                                                    const Batch bt) {
   pdl_chain();
   if (bt_skip(bt)) return;
@@ -3200,10 +3263,10 @@ __global__ void __launch_bounds__(MG_TPB) k_defect(const Lvl<double> F0, const L
   const int k = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y;
   if (k >= n || j >= n) return;
   const int i = bt_z(bt);
-  const double r = defect_at(F, n, i, j, k);
-  const_cast<float*>(Lf.rhs)[lid(Lf, i + 1, j + 1, k + 1)] = (float)r;
+  const float r = (float)defect_at(F, n, i, j, k);
+  const_cast<float*>(Lf.rhs)[lid(Lf, i + 1, j + 1, k + 1)] = r;
   // the FP32 correction starts from zero, ring included
-  zero_with_ring(Lf, n, i, j, k);
+  start_cell(Lf, rt, first, i, j, k, r);
 }
 
 // phi += the FP32 correction over the real cells and the ring.  With a split
@@ -3268,10 +3331,12 @@ static int dc_cycle(const Lvl<double>& F, std::vector<Lvl<float>>& lvf, const wf
   // the correction: no copy into the split layout and none back
   const bool sp = lvf.size() > 1 && split_resident(lvf[0], c);
   const Lvl<float> Lf = sp ? split_view(lvf[0]) : lvf[0];
-  WF_CK(launch_k(k_defect, cells3(n, n, n), cell_block(), 0, s, F, Lf));
+  const bool first = sp || (lvf.size() > 1 && relax_by_launches(lvf[0], c.n_pre));
+  WF_CK(launch_chain(k_defect, cells3(n, n, n), cell_block(), 0, s, F, Lf, first ? 1 : 0,
+                     ap_recip(Lf)));
   WF_CKL("k_defect");
-  WF_TRY(vcycle<float>(lvf, c, s, sp, sp, sp));
-  WF_CK(launch_k(k_correct, cells3(m, m, m), cell_block(), 0, s, F, Lf));
+  WF_TRY(vcycle<float>(lvf, c, s, sp, sp, sp, first));
+  WF_CK(launch_chain(k_correct, cells3(m, m, m), cell_block(), 0, s, F, Lf));
   WF_CKL("k_correct");
   return WF_OK;
 }
@@ -3379,7 +3444,7 @@ int mg_solve(const wf_case& c, cudaStream_t s) {
   const bool keep = split_resident(lv[0], c) && lv.size() > 1;
   for (int cyc = 0; cyc < c.n_vcycles; ++cyc)
     WF_TRY(vcycle<double>(lv, c, s, cyc > 0 && (c.n_pre > 0 || c.n_post > 0),
-                          keep && cyc > 0, keep && cyc + 1 < c.n_vcycles));
+                          keep && cyc > 0, keep && cyc + 1 < c.n_vcycles, false, cyc == 0));
   return WF_OK;
 }
 
@@ -3572,17 +3637,21 @@ static int noalloc_addrs(NoallocAddrs* out) {
 // the V-cycle of multigrid.py:301-322 over a fixed array of level views
 static int vcycle_fixed(Lvl<double>* lv, int L, const wf_case& c, cudaStream_t s) {
   for (int l = 0; l < L; ++l) {
+    bool first = false;
     if (l > 0) {
-      // k_restrict also zeroes the coarse phi, ring included
+      first = l < L - 1 && relax_by_launches(lv[l], c.n_pre);
       WF_CK(launch_chain(k_restrict<double>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s,
-          lv[l - 1], const_cast<double*>(lv[l].rhs), lv[l], c.n_pre > 0 ? 1 : 0));
+          lv[l - 1], const_cast<double*>(lv[l].rhs), lv[l], c.n_pre > 0 ? 1 : 0, first ? 1 : 0,
+          ap_recip(lv[l])));
       WF_CKL("k_restrict");
     }
-    WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, false, l > 0, l == L - 1));
+    WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, false, l > 0, l == L - 1,
+                 first));
   }
   for (int l = L - 2; l >= 0; --l) {
-    WF_CK(launch_chain(k_prolong<double>, cells3(lv[l].n, lv[l].n, lv[l].n), cell_block(), 0, s, 
-        lv[l + 1], lv[l]));
+    const int half = c.n_post > 0 ? 1 : 0;
+    WF_CK(launch_chain(k_prolong<double>, prolong_grid(lv[l].n, half), cell_block(), 0, s,
+                       lv[l + 1], lv[l], half));
     WF_CKL("k_prolong");
     WF_TRY(relax(lv[l], c.n_post, s));
   }
