@@ -206,7 +206,8 @@ static int launch_rbgs(const Lvl<T>& L, int color, bool pre, cudaStream_t s) {
 // half-sweep's.  Left in the cell, its face-ring mirrors, and zero in the other
 // ring cells nearest to it, so that the real cells' threads together write
 // every cell of the (n+2)^3 array exactly once.  first 0: zeros.
-//   FIRST_FIGURES
+// With the prolongations' half (k_prolong), us per step: 80^3 692 -> 674, 80^3
+// mixed 673 -> 651, 128^3 mixed 1497 -> 1462, 256^3 FP64 8925 -> 8803.
 template <class T>
 __device__ __forceinline__ T first_value(const Lvl<T>& L, const ApRecip<T>& rt, int i, int j, int k,
                                          T r) {
@@ -394,16 +395,21 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong(const Lvl<T> C0, Lvl<T> F0, 
 static dim3 prolong_grid(int n, int half) { return cells3(n, n, half ? (n + 1) / 2 : n); }
 
 // the same prolongation with one thread per COARSE cell writing its 2x2x2
-// fine cells from the 27 coarse values around it, each loaded once (27 loads
-// for 8 outputs instead of 64); every output sums the same terms in the
-// same order as k_prolong, so the results are the same bits.  The 8 fine
-// values are loaded before the first store: the stores go through the same
-// pointer, so the compiler would otherwise issue each load after the
-// previous cell's store, eight dependent memory round trips per thread.
-// Loading them first is safe because each fine cell is written by this
-// thread only, and ring_mirror writes ring cells, which are never loaded.
-template <class T>
-__global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0, int half,
+// fine cells (HALF: the four of the colour) from the 27 coarse values around it;
+// every output sums the same terms in the same order as k_prolong, so the
+// results are the same bits.  At large sizes a thread takes `planes` cells along
+// i: two of three coarse planes stay in registers, and the next cell's nine
+// values and fine cells are on their way while this one is computed (a cell per
+// thread is one round of latency at a time, at two CTAs per SM).  us per solve of
+// two V-cycles, before / now: 128^3 FP64 952 / 945, mixed 922 / 911, 256^3 FP64
+// 5452 / 5369, mixed 4469 / 4377; 4 or 16 planes instead of up to 8: within 0.2 %.
+// The fine values are loaded before the first store: the stores go through the
+// same pointer, so the compiler would otherwise issue each load after the
+// previous cell's store.  Loading them first is safe because each fine cell is
+// written by this thread only, and ring_mirror writes ring cells, which are
+// never loaded.
+template <class T, bool HALF, bool MARCH>
+__global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0, int planes,
                                                      const Batch bt) {
   if (bt.tab) {
     pdl_chain();
@@ -414,65 +420,86 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0,
   const int nc = C.n;
   const int ck = blockIdx.x * 32 + threadIdx.x, cj = blockIdx.y * 8 + threadIdx.y;
   const bool on = ck < nc && cj < nc;
-  const int ci = bt_z(bt);
+  const int ci0 = MARCH ? bt_z(bt) * planes : bt_z(bt);
+  const int ci1 = MARCH ? min(nc, ci0 + planes) : ci0 + 1;
+  // a thread's fine cells relative to the first of them
+  const int k1 = F.split ? (int)(spos(2 * ck + 2, (F.n + 2) >> 1) -
+                                 spos(2 * ck + 1, (F.n + 2) >> 1)) : 1;
+  const int sI = (int)F.sI, sJ = (int)F.sJ;
+  T* fp = F.phi + lid(F, 2 * ci0 + 1, 2 * cj + 1, 2 * ck + 1);
+  auto takes = [](int e) { return !HALF || (((e >> 2) + (e >> 1) + e) & 1) == 0; };
+  auto at = [&](int e) { return (e >> 2) * sI + ((e >> 1) & 1) * sJ + (e & 1) * k1; };
   // the fine level was last written before the restriction out of it, at least
   // two launches ahead (pdl_chain)
-  long fc[2][2][2];
-  T fv[2][2][2];
+  T fv[8];
 #pragma unroll
-  for (int pi = 0; pi < 2; ++pi)
-#pragma unroll
-    for (int pj = 0; pj < 2; ++pj)
-#pragma unroll
-      for (int pk = 0; pk < 2; ++pk) {
-        fc[pi][pj][pk] = lid(F, 2 * ci + pi + 1, 2 * cj + pj + 1, 2 * ck + pk + 1);
-        fv[pi][pj][pk] =
-            on && !(half && ((pi + pj + pk) & 1)) ? __ldcg(F.phi + fc[pi][pj][pk]) : T(0);
-      }
+  for (int e = 0; e < 8; ++e)
+    if (takes(e)) fv[e] = on ? __ldcg(fp + at(e)) : T(0);
   if (!bt.tab) pdl_chain();
   if (!on) return;
   const int Hc = (nc + 2) >> 1;
-  long kq[3];
+  int kq[3];
 #pragma unroll
-  for (int q = 0; q < 3; ++q) kq[q] = C.split ? spos(ck + q, Hc) : (ck + q);
+  for (int q = 0; q < 3; ++q) kq[q] = C.split ? (int)spos(ck + q, Hc) : (ck + q);
+  const T* cp = C.phi + (long)ci0 * C.sI + (long)cj * C.sJ;
   T Q[3][3][3];   // coarse (ci-1+a, cj-1+b, ck-1+q), ring included
 #pragma unroll
   for (int a = 0; a < 3; ++a)
 #pragma unroll
     for (int b = 0; b < 3; ++b)
 #pragma unroll
-      for (int q = 0; q < 3; ++q)
-        Q[a][b][q] = C.phi[(long)(ci + a) * C.sI + (long)(cj + b) * C.sJ + kq[q]];
+      for (int q = 0; q < 3; ++q) Q[a][b][q] = cp[a * C.sI + b * C.sJ + kq[q]];
+  for (int ci = ci0; ci < ci1; ++ci) {
+    T qn[3][3], fn[8];
+    if (MARCH && ci + 1 < ci1) {
 #pragma unroll
-  for (int pi = 0; pi < 2; ++pi)
+      for (int b = 0; b < 3; ++b)
 #pragma unroll
-    for (int pj = 0; pj < 2; ++pj)
+        for (int q = 0; q < 3; ++q) qn[b][q] = cp[3 * C.sI + b * C.sJ + kq[q]];
 #pragma unroll
-      for (int pk = 0; pk < 2; ++pk) {
-        if (half && ((pi + pj + pk) & 1)) continue;
-        const T wx0 = pi == 0 ? T(0.25) : T(0.75);
-        const T wy0 = pj == 0 ? T(0.25) : T(0.75);
-        const T wz0 = pk == 0 ? T(0.25) : T(0.75);
-        T acc = T(0);
+      for (int e = 0; e < 8; ++e)
+        if (takes(e)) fn[e] = __ldcg(fp + 2 * sI + at(e));
+    }
 #pragma unroll
-        for (int di = 0; di < 2; ++di) {
-          const T wxi = di == 0 ? wx0 : T(1) - wx0;
+    for (int e = 0; e < 8; ++e) {
+      if (!takes(e)) continue;
+      const int pi = e >> 2, pj = (e >> 1) & 1, pk = e & 1;
+      const T wx0 = pi == 0 ? T(0.25) : T(0.75);
+      const T wy0 = pj == 0 ? T(0.25) : T(0.75);
+      const T wz0 = pk == 0 ? T(0.25) : T(0.75);
+      T acc = T(0);
 #pragma unroll
-          for (int dj = 0; dj < 2; ++dj) {
-            const T wyj = dj == 0 ? wy0 : T(1) - wy0;
+      for (int di = 0; di < 2; ++di) {
+        const T wxi = di == 0 ? wx0 : T(1) - wx0;
 #pragma unroll
-            for (int dk = 0; dk < 2; ++dk) {
-              const T wzk = dk == 0 ? wz0 : T(1) - wz0;
-              acc = acc + wxi * wyj * wzk * Q[pi + di][pj + dj][pk + dk];
-            }
+        for (int dj = 0; dj < 2; ++dj) {
+          const T wyj = dj == 0 ? wy0 : T(1) - wy0;
+#pragma unroll
+          for (int dk = 0; dk < 2; ++dk) {
+            const T wzk = dk == 0 ? wz0 : T(1) - wz0;
+            acc = acc + wxi * wyj * wzk * Q[pi + di][pj + dj][pk + dk];
           }
         }
-        const int i = 2 * ci + pi, j = 2 * cj + pj, k = 2 * ck + pk;
-        const long c = fc[pi][pj][pk];
-        const T x = fv[pi][pj][pk] + acc;
-        F.phi[c] = x;
-        if (!F.split) ring_mirror(F, i, j, k, c, x);
       }
+      T* c = fp + at(e);
+      const T x = fv[e] + acc;
+      *c = x;
+      if (!F.split) ring_mirror(F, 2 * ci + pi, 2 * cj + pj, 2 * ck + pk, c - F.phi, x);
+    }
+    if (!MARCH) return;
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        Q[0][b][q] = Q[1][b][q];
+        Q[1][b][q] = Q[2][b][q];
+        Q[2][b][q] = qn[b][q];
+      }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) fv[e] = fn[e];
+    cp += C.sI;
+    fp += 2 * sI;
+  }
 }
 
 // ---- a whole relax() of a small level inside one CTA's shared memory ------
@@ -3166,8 +3193,14 @@ static int vcycle(std::vector<Lvl<T>>& lv, const wf_case& c, cudaStream_t s,
     // fine levels from 64: one thread per coarse cell (fewer loads); smaller
     // ones keep one thread per fine cell (more threads in flight)
     if (lv[l].n >= 64 && (lv[l].n & 1) == 0) {
-      WF_CK(launch_chain(k_prolong8<T>, cells3(lv[l + 1].n, lv[l + 1].n, lv[l + 1].n), cell_block(),
-                     0, s, vw[l + 1], vw[l], half));
+      // planes per thread: as many as leave about 1000 CTAs (7 per SM)
+      const int nc = lv[l + 1].n;
+      dim3 g = cells3(nc, nc, nc);
+      const int planes = std::max(1, std::min(8, (int)(g.x * g.y * g.z / 1000)));
+      g.z = (nc + planes - 1) / planes;
+      auto kern = half ? (planes > 1 ? k_prolong8<T, true, true> : k_prolong8<T, true, false>)
+                       : (planes > 1 ? k_prolong8<T, false, true> : k_prolong8<T, false, false>);
+      WF_CK(launch_chain(kern, g, cell_block(), 0, s, vw[l + 1], vw[l], planes));
       WF_CKL("k_prolong8");
     } else {
       WF_CK(launch_chain(k_prolong<T>, prolong_grid(lv[l].n, half), cell_block(), 0, s, vw[l + 1],
