@@ -77,13 +77,8 @@ __device__ __forceinline__ double warp_max(double v) {
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
   return v;
 }
-__device__ __forceinline__ double warp_min(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, o));
-  return v;
-}
 
-// block-wide max / min; every thread gets the result (blockDim <= 1024)
+// block-wide max; every thread gets the result (blockDim <= 1024)
 __device__ __forceinline__ double block_max(double v, double* sm) {
   v = warp_max(v);
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -93,19 +88,6 @@ __device__ __forceinline__ double block_max(double v, double* sm) {
   __syncthreads();
   v = (threadIdx.x < nw) ? sm[threadIdx.x] : 0.0;
   if (w == 0) v = warp_max(v);
-  if (threadIdx.x == 0) sm[0] = v;
-  __syncthreads();
-  return sm[0];
-}
-__device__ __forceinline__ double block_min(double v, double* sm, double ident) {
-  v = warp_min(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  const int nw = (blockDim.x + 31) >> 5;
-  __syncthreads();
-  if (l == 0) sm[w] = v;
-  __syncthreads();
-  v = (threadIdx.x < nw) ? sm[threadIdx.x] : ident;
-  if (w == 0) v = warp_min(v);
   if (threadIdx.x == 0) sm[0] = v;
   __syncthreads();
   return sm[0];

@@ -190,10 +190,11 @@ __global__ void __launch_bounds__(RBGS_TPB) k_rbgs(const Lvl<T> L0, int color, i
 }
 
 template <class T>
-static int launch_rbgs(const Lvl<T>& L, int color, bool pre, cudaStream_t s) {
+static int launch_rbgs(const Lvl<T>& L, int color, bool pre, const ApRecip<T>& rt,
+                       cudaStream_t s) {
   const int nh = (L.n + 1) / 2;
   WF_CK(launch_chain(k_rbgs<T>, dim3((L.n * nh + RBGS_TPB - 1) / RBGS_TPB, 1, L.n), RBGS_TPB, 0, s,
-                     L, color, pre ? 1 : 0, 1.0f / (float)nh, ap_recip(L)));
+                     L, color, pre ? 1 : 0, 1.0f / (float)nh, rt));
   WF_CKL("k_rbgs");
   return WF_OK;
 }
@@ -401,7 +402,7 @@ static dim3 prolong_grid(int n, int half) { return cells3(n, n, half ? (n + 1) /
 // i: two of three coarse planes stay in registers, and the next cell's nine
 // values and fine cells are on their way while this one is computed (a cell per
 // thread is one round of latency at a time, at two CTAs per SM).  us per solve of
-// two V-cycles, before / now: 128^3 FP64 952 / 945, mixed 922 / 911, 256^3 FP64
+// four V-cycles, before / now: 128^3 FP64 952 / 945, mixed 922 / 911, 256^3 FP64
 // 5452 / 5369, mixed 4469 / 4377; 4 or 16 planes instead of up to 8: within 0.2 %.
 // The fine values are loaded before the first store: the stores go through the
 // same pointer, so the compiler would otherwise issue each load after the
@@ -486,19 +487,20 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0,
       *c = x;
       if (!F.split) ring_mirror(F, 2 * ci + pi, 2 * cj + pj, 2 * ck + pk, c - F.phi, x);
     }
-    if (!MARCH) return;
+    if constexpr (MARCH) {
 #pragma unroll
-    for (int b = 0; b < 3; ++b)
+      for (int b = 0; b < 3; ++b)
 #pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        Q[0][b][q] = Q[1][b][q];
-        Q[1][b][q] = Q[2][b][q];
-        Q[2][b][q] = qn[b][q];
-      }
+        for (int q = 0; q < 3; ++q) {
+          Q[0][b][q] = Q[1][b][q];
+          Q[1][b][q] = Q[2][b][q];
+          Q[2][b][q] = qn[b][q];
+        }
 #pragma unroll
-    for (int e = 0; e < 8; ++e) fv[e] = fn[e];
-    cp += C.sI;
-    fp += 2 * sI;
+      for (int e = 0; e < 8; ++e) fv[e] = fn[e];
+      cp += C.sI;
+      fp += 2 * sI;
+    }
   }
 }
 
@@ -2147,7 +2149,8 @@ static int apply_coarse_op(const Lvl<T>& L, const T* op, T* part, cudaStream_t s
   WF_CK(launch_chain(k_cop_out<T>, (P.M + 255) / 256, 256, 0, s, (const T*)Y, prod, P.nrep, L));
   WF_CKL("k_cop_out");
   // the rhs was written before k_cop_vg
-  for (int color = 0; color < 2; ++color) WF_TRY(launch_rbgs(L, color, true, s));
+  const ApRecip<T> rt = ap_recip(L);
+  for (int color = 0; color < 2; ++color) WF_TRY(launch_rbgs(L, color, true, rt, s));
   return WF_OK;
 }
 
@@ -3053,7 +3056,7 @@ static bool relax_by_launches(const Lvl<T>& L, int nsweeps) {
   // 20^3 / 24^3 in one CTA 20.3 / 27.5 us, by launches 13.7 / 14.0 (16^3: 8.5 and
   // 13.5).  Not FP32, whose last bit the quotient in place of the reciprocal
   // would change.
-  if (L.n <= 24 && L.n % 4 == 0 && !(sizeof(T) == 8 && L.n >= 20)) return false;
+  if (L.n <= 24 && L.n % 4 == 0) return sizeof(T) == 8 && L.n >= 20;
   if (L.tmp && (L.n & 1) == 0 && L.n >= split_min_n()) return false;
   return batch_ctx().tab || !(mid_p2p_enabled() || (L.tmp && L.n >= sweep2_min_n()) ||
                               (L.gbar && L.n >= persist_min_n()));
@@ -3063,8 +3066,9 @@ static bool relax_by_launches(const Lvl<T>& L, int nsweeps) {
 template <class T>
 static int launch_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready,
                          bool first) {
+  const ApRecip<T> rt = ap_recip(L);
   for (int h = first ? 1 : 0; h < 2 * nsweeps; ++h)
-    WF_TRY(launch_rbgs(L, h & 1, h > (first ? 1 : 0) || rhs_ready, s));
+    WF_TRY(launch_rbgs(L, h & 1, h > (first ? 1 : 0) || rhs_ready, rt, s));
   return WF_OK;
 }
 
@@ -3113,8 +3117,9 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
       WF_TRY(launch_sweep2<T>(L.tmp, L.tI, L.tJ, L.phi, L.sI, L.sJ, L, ring, s));
     }
     if (nsweeps & 1) {
-      WF_TRY(launch_rbgs(L, 0, false, s));
-      WF_TRY(launch_rbgs(L, 1, true, s));
+      const ApRecip<T> rt = ap_recip(L);
+      WF_TRY(launch_rbgs(L, 0, false, rt, s));
+      WF_TRY(launch_rbgs(L, 1, true, rt, s));
     }
     return WF_OK;
   }
