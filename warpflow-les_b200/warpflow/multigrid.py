@@ -30,7 +30,8 @@ the cells (``wf_mg_build_coarse_op``) and a closing sweep, built once per
 (size, spacing, n_coarse, precision) and shared by every Multigrid of the
 process; each instance keeps its own partial-sum scratch.  Where the
 coarsest edge is not 4..24 in steps of 4, n_coarse < 2, or the operator
-would exceed ``COARSE_OP_MAX_BYTES``, the sweeps run as before.
+would exceed ``COARSE_OP_MAX_BYTES``, the sweeps run: in FP64 at even edges
+10..32 as a polynomial of the sweep map, else one by one.
 """
 from __future__ import annotations
 
