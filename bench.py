@@ -147,8 +147,7 @@ def load_peaks():
 
 # DRAM bytes per launch of the dominant kernels, from the ncu captures
 # summarised under profiles/ (dram__bytes_read.sum + dram__bytes_write.sum)
-NCU_TRAFFIC = {("k_rbgs_split", 256): (189163264, "profiles/rbgs_split_256_full.md"),
-               ("k_rbgs_split", 80): (5156864, "profiles/rbgs_split_80_full.md"),
+NCU_TRAFFIC = {("split half-sweep", 256): (183700000, "profiles/step256_launches.md"),
                ("coarse", 20): (172032, "profiles/coarse_p2p_20_full.md")}
 
 
@@ -225,7 +224,7 @@ def _split_roofline(mg, n, peak, peak_kind):
     lev0 = mg.levels[0]
     lev0.rhs.assign(np.random.default_rng(7).standard_normal(lev0.shape))
     t = (_timed_relax(mg, 0, 12, 20) - _timed_relax(mg, 0, 6, 20)) / 12
-    return _roof("k_rbgs_split (level-0 half-sweep, FP64)", ("k_rbgs_split", n),
+    return _roof("split half-sweep (level 0, FP64)", ("split half-sweep", n),
                  1.5 * n ** 3 * 8, t, peak, peak_kind)
 
 
