@@ -108,7 +108,9 @@ typedef struct wf_case {
   void* mg_tmp[WF_MAX_LEVELS];    /* optional scratch of 2*(n_l+2)^3 elements per level
                                      (level 0 included, element type of the level): large
                                      levels relax on row-parity-split copies of phi and rhs
-                                     held there; NULL = relax in place */
+                                     held there; NULL = relax in place.  Any
+                                     element-aligned address serves; one aligned to two
+                                     elements also lets levels from 144 relax in pairs */
   wf_scalars* sc;                 /* device scalar block */
   void* mg_cop;                   /* optional coarse-level operator (may be shared
                                      by cases), see wf_mg_build_coarse_op; NULL = sweeps */

@@ -80,6 +80,9 @@ struct BatchCtx {
   const CasePtrs* tab = nullptr;
   int ncases = 1;
   int skip = 0;
+  // per level, the OR of the low address bits of every case's mg_tmp: the
+  // alignment that a kernel of the bucket may count on
+  uint8_t tmp_bits[WF_MAX_LEVELS] = {};
 };
 BatchCtx& batch_ctx();
 

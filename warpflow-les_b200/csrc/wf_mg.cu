@@ -2579,8 +2579,10 @@ static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_r
   const ApRecip<T> rt = ap_recip(L);
   const bool set = launch_shape_set(SHAPE_SPLIT, n);
   const bool flat = n < FLAT_MAX_N && !set;
+  const BatchCtx& bc = batch_ctx();
+  const uintptr_t at = bc.tab ? bc.tmp_bits[L.role & 15] : (uintptr_t)L.tmp;   // every case's
   const bool pair = n >= PAIR_MIN_N && n % 4 == 0 && n <= 1024 && !set &&
-                    (uintptr_t)L.tmp % (2 * sizeof(T)) == 0;
+                    at % (2 * sizeof(T)) == 0;
   const int cells = n > 84 ? 2 : 1;
   const int planes = n >= 176 ? 4 : 2, prows = std::min(n >= 176 ? 2 : 4, MG_TPB / (n / 4));
   int cpt, rows, one;

@@ -44,14 +44,22 @@ BatchCtx& batch_ctx() {
   return ctx;
 }
 
-// Launches of this thread serve the bucket `tab` (ncases cases) for one
-// scope; tab null = one case.
+// Launches of this thread serve the bucket `tab` for one scope (rows: the
+// host's copy of that table); tab null = one case.
 struct BatchScope {
   BatchCtx prev;
-  BatchScope(const CasePtrs* tab, int ncases, int skip) : prev(batch_ctx()) {
-    batch_ctx().tab = tab;
-    batch_ctx().ncases = tab ? ncases : 1;
-    batch_ctx().skip = tab ? skip : 0;
+  BatchScope(const CasePtrs* tab, const std::vector<CasePtrs>& rows, int skip)
+      : prev(batch_ctx()) {
+    BatchCtx bc;
+    if (tab) {
+      bc.tab = tab;
+      bc.ncases = (int)rows.size();
+      bc.skip = skip;
+      for (const CasePtrs& p : rows)
+        for (int l = 0; l < WF_MAX_LEVELS; ++l)
+          bc.tmp_bits[l] |= (uint8_t)((uintptr_t)p.mg_tmp[l] & 15);
+    }
+    batch_ctx() = bc;
   }
   ~BatchScope() { batch_ctx() = prev; }
 };
@@ -160,12 +168,12 @@ struct wf_stepper {
 // Append one case's step to graph g as an independent branch (its first
 // nodes have no dependencies): the prologue, a WHILE node over calmas and
 // an IF node holding the multigrid part, then the epilogue.  counts gets the
-// launches of each part.  With `tab` (ncases rows, c = the first case) the
+// launches of each part.  With `tab` (its rows in `rows`, c = the first case) the
 // branch steps the whole bucket: every launch serves every case, the
 // multigrid part only the cases whose own loop runs it this iteration, and
 // the loop runs while any case's loop does.
 static int append_step(cudaGraph_t g, const wf_case& c, int32_t counts[4],
-                       const CasePtrs* tab = nullptr, int ncases = 1) {
+                       const CasePtrs* tab = nullptr, const std::vector<CasePtrs>& rows = {}) {
   cudaStream_t cap;
   WF_CK(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
   int rc = WF_OK;
@@ -177,7 +185,7 @@ static int append_step(cudaGraph_t g, const wf_case& c, int32_t counts[4],
     if (e != cudaSuccess) { rc = cuda_fail(e, "cudaStreamBeginCaptureToGraph"); break; }
     long l0 = g_launches;
     {
-      BatchScope bs(tab, ncases, 0);
+      BatchScope bs(tab, rows, 0);
       rc = step_prologue(c, cap);
     }
     counts[0] = (int32_t)(g_launches - l0);
@@ -204,7 +212,7 @@ static int append_step(cudaGraph_t g, const wf_case& c, int32_t counts[4],
       }
       l0 = g_launches;
       if (rc == WF_OK) {
-        BatchScope bs(tab, ncases, 0);
+        BatchScope bs(tab, rows, 0);
         rc = step_epilogue(c, cap);
       }
       counts[3] = (int32_t)(g_launches - l0);
@@ -222,7 +230,7 @@ static int append_step(cudaGraph_t g, const wf_case& c, int32_t counts[4],
     if (e != cudaSuccess) { rc = cuda_fail(e, "cudaStreamBeginCaptureToGraph(while)"); break; }
     l0 = g_launches;
     {
-      BatchScope bs(tab, ncases, 0);
+      BatchScope bs(tab, rows, 0);
       rc = launch_calmas(c, (unsigned long long)h_if, (unsigned long long)h_loop, cap);
     }
     counts[1] = (int32_t)(g_launches - l0);
@@ -256,7 +264,7 @@ static int append_step(cudaGraph_t g, const wf_case& c, int32_t counts[4],
     if (e != cudaSuccess) { rc = cuda_fail(e, "cudaStreamBeginCaptureToGraph(if)"); break; }
     l0 = g_launches;
     {
-      BatchScope bs(tab, ncases, 2);   // only cases whose loop runs the multigrid part
+      BatchScope bs(tab, rows, 2);   // only cases whose loop runs the multigrid part
       rc = step_mg_part(c, cap);
     }
     counts[2] = (int32_t)(g_launches - l0);
@@ -649,7 +657,7 @@ int wf_ensemble_create(const wf_case* cases, int32_t ncases, int32_t mode, wf_en
       e = cudaMemcpy(tab, rows.data(), rows.size() * sizeof(CasePtrs), cudaMemcpyHostToDevice);
       if (e != cudaSuccess) { rc = cuda_fail(e, "cudaMemcpy(bucket table)"); break; }
       int32_t counts[4] = {0, 0, 0, 0};
-      rc = append_step(en->graph, cases[b[0]], counts, (const CasePtrs*)tab, (int)b.size());
+      rc = append_step(en->graph, cases[b[0]], counts, (const CasePtrs*)tab, rows);
       en->counts.insert(en->counts.end(), counts, counts + 4);
     }
   } else {
@@ -686,7 +694,7 @@ int wf_mg_solve_bucket(const wf_case* cases, int32_t ncases, void* table, void* 
   WF_CK(cudaMemcpyAsync(table, rows.data(), rows.size() * sizeof(CasePtrs),
                         cudaMemcpyHostToDevice, s));
   WF_CK(cudaStreamSynchronize(s));   // the rows live on this thread's stack
-  BatchScope bs((const CasePtrs*)table, ncases, 0);
+  BatchScope bs((const CasePtrs*)table, rows, 0);
   return mg_solve(cases[0], s);
 }
 
