@@ -2584,12 +2584,14 @@ static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_r
   const bool pair = n >= PAIR_MIN_N && n % 4 == 0 && n <= 1024 && !set &&
                     at % (2 * sizeof(T)) == 0;
   const int cells = n > 84 ? 2 : 1;
-  const int planes = n >= 176 ? 4 : 2, prows = std::min(n >= 176 ? 2 : 4, MG_TPB / (n / 4));
+  // k_rbgs_pair: a row of n / 4 threads, at most MG_TPB in a CTA
+  const int planes = n >= 176 ? 4 : 2;
+  const int prows = pair ? std::min(n >= 176 ? 2 : 4, MG_TPB / (n / 4)) : 1;
   int cpt, rows, one;
   launch_shape(SHAPE_SPLIT, n, &cpt, &rows, &one);   // cpt in {1, 2, 4, 8}, rows <= SPLIT_ROWS
   const dim3 grid((nh + 32 * cpt - 1) / (32 * cpt), (n + rows - 1) / rows, n);
   const dim3 fgrid((n * nh + MG_TPB * cells - 1) / (MG_TPB * cells), 1, n);
-  const dim3 pgrid((n + prows - 1) / std::max(1, prows), 1, (n + planes - 1) / planes);
+  const dim3 pgrid((n + prows - 1) / prows, 1, (n + planes - 1) / planes);
   auto kern = cpt == 8   ? k_rbgs_split<T, 8>
               : cpt == 4 ? k_rbgs_split<T, 4>
               : cpt == 2 ? k_rbgs_split<T, 2>
