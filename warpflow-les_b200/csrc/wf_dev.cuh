@@ -127,4 +127,23 @@ __device__ __forceinline__ T div_by_recip(T x, T d, T y) {
   return fma(r, y, q);
 }
 
+__device__ __forceinline__ bool finite_bits(double x) {
+  return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
+}
+__device__ __forceinline__ bool finite_bits(float x) {
+  return (__float_as_int(x) & 0x7f800000) != 0x7f800000;
+}
+
+// the same quotient where x may be infinite: the corrections turn an infinity
+// into a NaN, so the first product, which has the quotient's sign, stands
+template <class T>
+__device__ __forceinline__ T div_by_recip_inf(T x, T d, T y) {
+  const T q = x * y;
+  T r = fma(-q, d, x);
+  T p = fma(r, y, q);
+  r = fma(-p, d, x);
+  p = fma(r, y, p);
+  return finite_bits(q) ? p : q;
+}
+
 }  // namespace wf

@@ -146,7 +146,8 @@ static ApRecip<T> ap_recip(const Lvl<T>& L) {
 // (rnh = 1 / cells per row).  A launch of these small levels is a chain of
 // latencies (start, index arithmetic, one round of loads, the dependent FP64
 // operations, the store); everything that does not depend on the launch ahead
-// comes before the wait, and the quotient is the reciprocal form's.  us per
+// comes before the wait, and the quotient is the reciprocal form's, with an
+// infinite numerator kept (32^3 step 361 -> 362.5 us).  us per
 // half-sweep in a graph, before / now: 32^3 1.87 / 1.19, 40^3 2.12 / 1.30,
 // 48^3 2.07 / 1.45.  pre: the level's rhs was complete before the launch ahead
 // of this one (pdl_chain), so it may be read ahead of the wait.
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(RBGS_TPB) k_rbgs(const Lvl<T> L0, int color, i
   const T* phi = L.phi + c;
   const T s = aw * phi[-sI] + ae * phi[sI] + as * phi[-sJ] + an * phi[sJ] + ab * phi[-1] +
               at * phi[1];
-  const T x = div_by_recip(r - s, ap, y);
+  const T x = div_by_recip_inf(r - s, ap, y);
   L.phi[c] = x;
   ring_mirror(L, i, j, k, c, x);
 }
@@ -217,9 +218,9 @@ __device__ __forceinline__ T first_value(const Lvl<T>& L, const ApRecip<T>& rt, 
   const T aw = i > 0 ? L.ax : T(0), ae = i < n - 1 ? L.ax : T(0);
   const T as = j > 0 ? L.ay : T(0), an = j < n - 1 ? L.ay : T(0);
   const T ab = k > 0 ? L.az : T(0), at = k < n - 1 ? L.az : T(0);
-  return div_by_recip(r, -(aw + ae + as + an + ab + at),
-                      rt.y[9 * ((i > 0) + (i < n - 1)) + 3 * ((j > 0) + (j < n - 1)) + (k > 0) +
-                           (k < n - 1)]);
+  return div_by_recip_inf(r, -(aw + ae + as + an + ab + at),
+                          rt.y[9 * ((i > 0) + (i < n - 1)) + 3 * ((j > 0) + (j < n - 1)) +
+                               (k > 0) + (k < n - 1)]);
 }
 
 template <class T>
@@ -2249,6 +2250,15 @@ static int try_coarse_cluster(const Lvl<T>& L, int nsweeps, cudaStream_t s, int*
 // mirrors, which is what k_rbgs leaves in the ring after the last sweep.
 constexpr int SPLIT_ROWS = 8;  // rows (one warp each) per CTA
 
+// INF: an infinite numerator stays an infinity (div_by_recip_inf), as in
+// k_rbgs.  Levels below 80 cells in FP64 and 128 in FP32 keep to that; it costs
+// 0.6 % of an 80^3 FP64 step and 0.9 % of a 256^3 one, and larger levels go
+// without (an infinity becomes a NaN there).
+template <bool INF, class T>
+__device__ __forceinline__ T quotient(T x, T d, T y) {
+  return INF ? div_by_recip_inf(x, d, y) : div_by_recip(x, d, y);
+}
+
 // level phi (all (n+2)^3 cells) and rhs -> split copies sp, sr (dense strides);
 // first (with_rhs set): phi is zero and is not read, first_value takes its place
 template <class T>
@@ -2284,7 +2294,7 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
 // x = chunk of 32*CPT cells of the half-row, y = group of blockDim.y rows j
 // (at most SPLIT_ROWS; CPT and the rows are chosen per size), z = plane i.  All loads of a thread come before its stores: a half-sweep
 // reads only the other colour and rhs, which it does not write.
-template <class T, int CPT>
+template <class T, int CPT, bool INF>
 __global__ void __launch_bounds__(32 * SPLIT_ROWS)
     k_rbgs_split(const Lvl<T> L0, T* sp, const T* sr, int color, int pre,
                  const __grid_constant__ ApRecip<T> rt, const Batch bt) {
@@ -2338,7 +2348,7 @@ __global__ void __launch_bounds__(32 * SPLIT_ROWS)
       const T ab = k > 0 ? L.az : T(0), at = k < n - 1 ? L.az : T(0);
       const T ap = -(aw + ae + as + an + ab + at);
       const T s = aw * vw[u] + ae * ve[u] + as * vs[u] + an * vn[u] + ab * vb[u] + at * vt[u];
-      own[32 * u] = div_by_recip(vr[u] - s, ap, rt.y[pij + (k > 0) + (k < n - 1)]);
+      own[32 * u] = quotient<INF>(vr[u] - s, ap, rt.y[pij + (k > 0) + (k < n - 1)]);
     }
   }
 }
@@ -2432,7 +2442,7 @@ __global__ void __launch_bounds__(256)
 // (rnh = 1 / cells per half-row), CPT cells a thread
 constexpr int FLAT_MAX_N = 104;
 
-template <class T, int CPT>
+template <class T, int CPT, bool INF>
 __global__ void __launch_bounds__(MG_TPB)
     k_rbgs_flat(const Lvl<T> L0, T* sp, const T* sr, int color, int pre, const float rnh,
                 const __grid_constant__ ApRecip<T> rt, const Batch bt) {
@@ -2489,7 +2499,7 @@ __global__ void __launch_bounds__(MG_TPB)
     const T ap = -(aw + ae + as + an + ab + at);
     const T y = rt.y[pi + 3 * ((j > 0) + (j < n - 1)) + (k > 0) + (k < n - 1)];
     const T s = aw * vw[u] + ae * ve[u] + as * vs[u] + an * vn[u] + ab * vb[u] + at * vt[u];
-    sp[own[u]] = div_by_recip(x[u] - s, ap, y);
+    sp[own[u]] = quotient<INF>(x[u] - s, ap, y);
   }
 }
 
@@ -2592,11 +2602,13 @@ static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_r
   const dim3 grid((nh + 32 * cpt - 1) / (32 * cpt), (n + rows - 1) / rows, n);
   const dim3 fgrid((n * nh + MG_TPB * cells - 1) / (MG_TPB * cells), 1, n);
   const dim3 pgrid((n + prows - 1) / prows, 1, (n + planes - 1) / planes);
-  auto kern = cpt == 8   ? k_rbgs_split<T, 8>
-              : cpt == 4 ? k_rbgs_split<T, 4>
-              : cpt == 2 ? k_rbgs_split<T, 2>
-                         : k_rbgs_split<T, 1>;
-  auto kflat = cells == 2 ? k_rbgs_flat<T, 2> : k_rbgs_flat<T, 1>;
+  const bool inf = n < (sizeof(T) == 4 ? 128 : 80);
+  auto kern = cpt == 8   ? (inf ? k_rbgs_split<T, 8, true> : k_rbgs_split<T, 8, false>)
+              : cpt == 4 ? (inf ? k_rbgs_split<T, 4, true> : k_rbgs_split<T, 4, false>)
+              : cpt == 2 ? (inf ? k_rbgs_split<T, 2, true> : k_rbgs_split<T, 2, false>)
+                         : (inf ? k_rbgs_split<T, 1, true> : k_rbgs_split<T, 1, false>);
+  auto kflat = cells == 2 ? (inf ? k_rbgs_flat<T, 2, true> : k_rbgs_flat<T, 2, false>)
+                          : (inf ? k_rbgs_flat<T, 1, true> : k_rbgs_flat<T, 1, false>);
   for (int h = first ? 1 : 0; h < 2 * nsweeps; ++h) {
     // after the first of these launches, the launch ahead is a half-sweep
     const int pre = h > (first ? 1 : 0) || rhs_ready ? 1 : 0, color = h & 1, back = n >= 176 ? color : 0;
