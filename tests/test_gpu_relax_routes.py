@@ -1,5 +1,5 @@
 """The routes a relax can take, where they could part: split copies of the
-smallest edges, infinities."""
+smallest edges, infinities, a ring that was never set."""
 import os
 import subprocess
 import sys
@@ -73,3 +73,63 @@ def test_infinities_stay_infinities(n, sign):
     np.testing.assert_array_equal(got[~fin], ref[~fin])
     # 4 half-sweeps of a handful of roundings each
     assert np.abs(got[fin] - ref[fin]).max() <= 1e-14 * np.abs(ref[fin]).max()
+
+
+RING_EDGES = [11, 13, 14, 15, 17, 18, 19, 20, 21, 22, 23, 24]
+
+
+def _nan_ring(a, n):
+    out = np.full((n + 2,) * 3, np.nan)
+    out[1:-1, 1:-1, 1:-1] = a[1:-1, 1:-1, 1:-1]
+    return out
+
+
+@pytest.mark.parametrize("sweeps", [1, 6, 13])
+@pytest.mark.parametrize("n", RING_EDGES)
+def test_relax_needs_no_ring(n, sweeps):
+    """Up to 24 cells the ring of phi may hold anything: the same cells and the
+    same ring come out as with the mirrors in it, from the host and in a graph."""
+    import torch
+    mg = _mg(n)
+    rng = np.random.default_rng(n)
+    phi = rng.standard_normal((n + 2,) * 3)
+    O.mg_refill(phi, n)
+    mg.levels[0].rhs.assign(rng.standard_normal((n + 2,) * 3))
+    real = np.s_[1:-1, 1:-1, 1:-1]
+    out = []
+    for start in (phi, _nan_ring(phi, n)):
+        mg.levels[0].phi.assign(start)
+        mg._relax(0, sweeps)
+        out.append(mg.levels[0].phi.numpy())
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            mg._relax(0, sweeps)
+        mg.levels[0].phi.assign(_nan_ring(phi, n))
+        g.replay()
+        s.synchronize()
+        out.append(mg.levels[0].phi.numpy())
+    assert np.isfinite(out[0]).all()
+    for o in out[1:]:
+        np.testing.assert_array_equal(o[real], out[0][real])
+        for sl in (np.s_[:, 1:-1, 1:-1], np.s_[1:-1, :, 1:-1], np.s_[1:-1, 1:-1, :]):
+            np.testing.assert_array_equal(o[sl], out[0][sl])
+
+
+@pytest.mark.parametrize("n,levels", [(14, 1), (14, 2), (18, 2), (20, 2), (24, 2), (24, 3),
+                                      (13, 1)])
+def test_vcycle_needs_no_ring(n, levels):
+    mg = _mg(n, levels)
+    rng = np.random.default_rng(n)
+    phi = rng.standard_normal((n + 2,) * 3)
+    O.mg_refill(phi, n)
+    mg.levels[0].rhs.assign(rng.standard_normal((n + 2,) * 3))
+    out = []
+    for start in (phi, _nan_ring(phi, n)):
+        mg.levels[0].phi.assign(start)
+        mg._vcycle()
+        out.append(mg.levels[0].phi.numpy()[1:-1, 1:-1, 1:-1])
+    assert np.isfinite(out[0]).all()
+    np.testing.assert_array_equal(out[0], out[1])

@@ -3505,10 +3505,43 @@ int mg_solve(const wf_case& c, cudaStream_t s) {
   return WF_OK;
 }
 
+__global__ void k_refill(Lvl<double> L) {
+  pdl_chain();
+  const int n = L.n;
+  const long tot = (long)n * n;
+  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < tot;
+       t += (long)gridDim.x * blockDim.x) {
+    const int a = 1 + (int)(t / n), b = 1 + (int)(t % n);
+    double* p = L.phi;
+    p[lid(L, 0, a, b)] = p[lid(L, 1, a, b)];
+    p[lid(L, n + 1, a, b)] = p[lid(L, n, a, b)];
+    p[lid(L, a, 0, b)] = p[lid(L, a, 1, b)];
+    p[lid(L, a, n + 1, b)] = p[lid(L, a, n, b)];
+    p[lid(L, a, b, 0)] = p[lid(L, a, b, 1)];
+    p[lid(L, a, b, n + 1)] = p[lid(L, a, b, n)];
+  }
+}
+
+static int refill(const Lvl<double>& L, cudaStream_t s) {
+  WF_CK(launch_k(k_refill, mg_blocks((long)L.n * L.n), MG_TPB, 0, s, L));
+  WF_CKL("k_refill");
+  return WF_OK;
+}
+
+// sweeps that run as launches of k_rbgs at an edge where one CTA or a cluster,
+// which do not read the ring, hold the level otherwise.  k_rbgs multiplies the
+// ring by zero, so a caller's phi0, whose ring may hold anything, gets its mirrors
+// first.
+static bool launches_meet_ring(int n, int nsweeps) {
+  if (nsweeps < 1 || n <= 10 || n > 24) return false;
+  return nsweeps <= 12 ? n % 4 != 0 || n >= 20 : n % 2 != 0;
+}
+
 int mg_vcycle_pair(const wf_case& c, double* phi0, const double* rhs0, cudaStream_t s) {
   const long m = c.n + 2;
   std::vector<Lvl<double>> lv;
   WF_TRY(build_levels<double>(c, phi0, rhs0, m * m, m, lv));
+  if (launches_meet_ring(c.n, c.nlev > 1 ? c.n_pre : c.n_coarse)) WF_TRY(refill(lv[0], s));
   return vcycle<double>(lv, c, s);
 }
 
@@ -3517,6 +3550,7 @@ int mg_relax_pair(const wf_case& c, double* phi0, const double* rhs0, int nsweep
   const long m = c.n + 2;
   std::vector<Lvl<double>> lv;
   WF_TRY(build_levels<double>(c, phi0, rhs0, m * m, m, lv));
+  if (launches_meet_ring(c.n, nsweeps)) WF_TRY(refill(lv[0], s));
   return relax<double>(lv[0], nsweeps, s);
 }
 
@@ -3548,30 +3582,11 @@ int mg_coarse_solve_pair(const wf_case& c, double* phi, const double* rhs, cudaS
   return relax<double>(L, c.n_coarse, s, false, true);
 }
 
-__global__ void k_refill(Lvl<double> L) {
-  pdl_chain();
-  const int n = L.n;
-  const long tot = (long)n * n;
-  for (long t = blockIdx.x * (long)blockDim.x + threadIdx.x; t < tot;
-       t += (long)gridDim.x * blockDim.x) {
-    const int a = 1 + (int)(t / n), b = 1 + (int)(t % n);
-    double* p = L.phi;
-    p[lid(L, 0, a, b)] = p[lid(L, 1, a, b)];
-    p[lid(L, n + 1, a, b)] = p[lid(L, n, a, b)];
-    p[lid(L, a, 0, b)] = p[lid(L, a, 1, b)];
-    p[lid(L, a, n + 1, b)] = p[lid(L, a, n, b)];
-    p[lid(L, a, b, 0)] = p[lid(L, a, b, 1)];
-    p[lid(L, a, b, n + 1)] = p[lid(L, a, b, n)];
-  }
-}
-
 int mg_refill_pair(const wf_case& c, double* phi0, cudaStream_t s) {
   const long m = c.n + 2;
   std::vector<Lvl<double>> lv;
   WF_TRY(build_levels<double>(c, phi0, phi0, m * m, m, lv));
-  WF_CK(launch_k(k_refill, mg_blocks((long)c.n * c.n), MG_TPB, 0, s, lv[0]));
-  WF_CKL("k_refill");
-  return WF_OK;
+  return refill(lv[0], s);
 }
 
 int mg_residual_max_pair(const wf_case& c, const double* phi0, const double* rhs0,
