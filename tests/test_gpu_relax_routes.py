@@ -1,5 +1,5 @@
 """The routes a relax can take, where they could part: split copies of the
-smallest edges, infinities, a ring that was never set."""
+smallest edges, infinities, a ring that was never set, one CTA and launches."""
 import os
 import subprocess
 import sys
@@ -133,3 +133,56 @@ def test_vcycle_needs_no_ring(n, levels):
         out.append(mg.levels[0].phi.numpy()[1:-1, 1:-1, 1:-1])
     assert np.isfinite(out[0]).all()
     np.testing.assert_array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("n", [11, 12, 14, 15, 16, 17, 20, 24])
+def test_one_sweep_at_a_time_equals_all(n):
+    """One CTA, launches and clusters: 13 sweeps at once, one at a time, and
+    recorded in a graph are the same bits off the multiples of four, and the
+    same to rounding on them (which multiply by the diagonal's reciprocal)."""
+    import torch
+    mg = _mg(n)
+    rng = np.random.default_rng(n)
+    phi = rng.standard_normal((n + 2,) * 3)
+    mg.levels[0].rhs.assign(rng.standard_normal((n + 2,) * 3))
+    out = []
+    for parts in ((13,), (1,) * 13, (6, 7)):
+        mg.levels[0].phi.assign(phi)
+        for k in parts:
+            mg._relax(0, k)
+        out.append(mg.levels[0].phi.numpy()[1:-1, 1:-1, 1:-1])
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            mg._relax(0, 13)
+        mg.levels[0].phi.assign(phi)
+        g.replay()
+        s.synchronize()
+        out.append(mg.levels[0].phi.numpy()[1:-1, 1:-1, 1:-1])
+    for o in out[1:]:
+        if n % 4:
+            np.testing.assert_array_equal(o, out[0])
+        else:   # 26 half-sweeps of two roundings each from the other form
+            assert np.abs(o - out[0]).max() <= 26 * 4.4e-16 * np.abs(out[0]).max()
+
+
+def test_odd_coarsest_level_from_the_host_and_in_a_graph():
+    """The 300 sweeps of an 11^3 coarsest level: one launch each when the host
+    issues them, 600 in a graph, where a launch costs less; the same fields."""
+    import ctypes
+    from warpflow import FlowSolver, _abi, build_topology
+    counts, fields = [], []
+    for mode in ("host", "graph"):
+        sol = FlowSolver(make_cfg(44), build_topology(make_cfg(44)), "cuda:0", step_mode=mode)
+        for _ in range(2):
+            sol.step()
+        c = (ctypes.c_int32 * 4)()
+        _abi.call("wf_stepper_launch_counts", sol._stepper, c)
+        counts.append(c[2])
+        fields.append([sol.f[k].numpy() for k in ("u", "v", "w", "p", "pp")])
+        sol.close()
+    assert counts[0] < 300 and counts[1] - counts[0] == 4 * 599
+    for a, b in zip(*fields):
+        np.testing.assert_array_equal(a, b)

@@ -510,7 +510,7 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0,
 // ring is not needed there because every ring term has a zero coefficient.
 // After the last sweep the interior and the face rings go back to global.
 template <class T>
-__global__ void __launch_bounds__(512) k_relax_smem(Lvl<T> L0, int nsweeps, const Batch bt) {
+__global__ void __launch_bounds__(1024) k_relax_smem(Lvl<T> L0, int nsweeps, const Batch bt) {
   pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
@@ -3091,6 +3091,40 @@ static int launch_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_
   return WF_OK;
 }
 
+static bool capturing(cudaStream_t s) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+    cudaGetLastError();   // e.g. the legacy stream while another one records
+    return false;
+  }
+  return st == cudaStreamCaptureStatusActive;
+}
+
+// Whether one CTA sweeps the level in shared memory (k_relax_smem) rather than a
+// launch per half-sweep (the same bits).  A launch costs 1.1 us in a graph and
+// 2.5 us from the host.  In a graph one CTA is up to 10: us for 6 sweeps, one
+// CTA / launches: 10^3 11.5 / 15.1, 11^3 18.1 / 15.1, 14^3 25.2 / 13.6, 22^3 78 /
+// 14.  From the host one CTA is up to 15, and to 17 for few sweeps: us for 12 / 40 /
+// 300 sweeps, one CTA, launches: 11^3 44 / 115 / 746, 101 / 297 / 1475, 13^3 56 / 145
+// / 972, 103 / 212 / 1463, 15^3 69 / 183 / 1235, 88 / 241 / 1695, 17^3 88 / 246 /
+// 1694, 99 / 279 / 1470.
+static bool one_cta(int n, int nsweeps, cudaStream_t s) {
+  return n <= 10 || (n <= (nsweeps <= 100 ? 17 : 15) && !capturing(s));
+}
+
+template <class T>
+static int launch_relax_smem(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
+  const int n3 = L.n * L.n * L.n;
+  const int tpb = std::min(1024, std::max(32, (n3 / 2 + 31) / 32 * 32));
+  const size_t sb = 2 * (size_t)n3 * sizeof(T);
+  if (sb > 48 * 1024)
+    WF_CK(cudaFuncSetAttribute(k_relax_smem<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)sb));
+  WF_CK(launch_chain(k_relax_smem<T>, 1, tpb, sb, s, L, nsweeps));
+  WF_CKL("k_relax_smem");
+  return WF_OK;
+}
+
 // rhs_ready: the level's rhs is unchanged since its last relax, so a split
 // copy of it made then can be reused
 // zero: the level's phi is zero (a level after the restriction)
@@ -3147,16 +3181,7 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
     WF_TRY(launch_relax_persist<T>(L, nsweeps, s, &done));
     if (done) return WF_OK;
   }
-  // up to 10 one CTA sweeps in shared memory, from 11 each half-sweep is a
-  // launch (the same bits).  us for 6 sweeps, one CTA / launches: 10^3 11.5 /
-  // 15.1, 11^3 18.1 / 15.1, 14^3 25.2 / 13.6, 18^3 45.0 / 13.7, 22^3 78.0 / 14.0
-  if (L.n <= 10) {
-    const int n3 = L.n * L.n * L.n;
-    const int tpb = (n3 / 2 + 31) / 32 * 32;
-    WF_CK(launch_chain(k_relax_smem<T>, 1, std::max(32, tpb), 2 * n3 * sizeof(T), s, L, nsweeps));
-    WF_CKL("k_relax_smem");
-    return WF_OK;
-  }
+  if (one_cta(L.n, nsweeps, s)) return launch_relax_smem(L, nsweeps, s);
   return launch_sweeps(L, nsweeps, s, rhs_ready, false);
 }
 
@@ -3545,13 +3570,32 @@ int mg_vcycle_pair(const wf_case& c, double* phi0, const double* rhs0, cudaStrea
   return vcycle<double>(lv, c, s);
 }
 
+// A relax on its own, not inside a V-cycle's chain of launches.  From the host
+// a launch costs 2.5 us whatever it does, so what needs few of them is preferred:
+// up to 12 sweeps in one CTA where that was measured no slower (us for 6 / 12
+// sweeps, launches, one CTA: 11^3 59 / 101, 31 / 44; 15^3 50 / 88, 45 / 69; from
+// three sweeps 20^3 42 / 72, 31 / 44 and 24^3 43 / 72, 38 / 57), and no copies into
+// the split layout for one or two sweeps (64^3, one sweep: 22 -> 18).
+static int relax_direct(const Lvl<double>& L, int nsweeps, cudaStream_t s) {
+  if (nsweeps <= 0) return WF_OK;
+  int rc = WF_OK;
+  if (nsweeps > 2 && nsweeps <= 12 && (L.n == 20 || L.n == 24) &&
+      try_coarse<double>(L, nsweeps, s, false, false, &rc))
+    return rc;
+  if (nsweeps <= 12 && L.n > 10 && L.n % 4 != 0 && one_cta(L.n, nsweeps, s))
+    return launch_relax_smem(L, nsweeps, s);
+  if (launches_meet_ring(L.n, nsweeps)) WF_TRY(refill(L, s));
+  Lvl<double> R = L;
+  if (nsweeps <= 2 && L.n >= 64 && L.n < 80) R.tmp = nullptr;
+  return relax<double>(R, nsweeps, s);
+}
+
 int mg_relax_pair(const wf_case& c, double* phi0, const double* rhs0, int nsweeps,
                   cudaStream_t s) {
   const long m = c.n + 2;
   std::vector<Lvl<double>> lv;
   WF_TRY(build_levels<double>(c, phi0, rhs0, m * m, m, lv));
-  if (launches_meet_ring(c.n, nsweeps)) WF_TRY(refill(lv[0], s));
-  return relax<double>(lv[0], nsweeps, s);
+  return relax_direct(lv[0], nsweeps, s);
 }
 
 // the coarsest-level solve of a V-cycle on an explicit (n_c+2)^3 pair: phi
