@@ -3623,7 +3623,7 @@ int mg_coarse_solve_pair(const wf_case& c, double* phi, const double* rhs, cudaS
   WF_CKL("k_zero");
   if (c.mg_cop && c.mg_cop_part && !c.mg_fp32 && c.n_coarse >= 2 && cop_size_ok(L.n))
     return apply_coarse_op<double>(L, (const double*)c.mg_cop, (double*)c.mg_cop_part, s);
-  return relax<double>(L, c.n_coarse, s, false, true);
+  return relax<double>(L, c.n_coarse, s, false, true, true);
 }
 
 int mg_refill_pair(const wf_case& c, double* phi0, cudaStream_t s) {
