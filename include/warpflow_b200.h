@@ -88,6 +88,8 @@ typedef struct wf_scalars {
   int32_t bflags;     /* bucket stepping: OR of the cases' loop decisions */
 } wf_scalars;
 
+#define WF_MG_COP_SWEEPS ((void*)1)   /* wf_case.mg_cop: see there */
+
 /* One cavity case: geometry, physics, numerics and the caller's buffers. */
 typedef struct wf_case {
   int32_t n;            /* cells per axis */
@@ -113,7 +115,11 @@ typedef struct wf_case {
                                      elements also lets levels from 144 relax in pairs */
   wf_scalars* sc;                 /* device scalar block */
   void* mg_cop;                   /* optional coarse-level operator (may be shared
-                                     by cases), see wf_mg_build_coarse_op; NULL = sweeps */
+                                     by cases), see wf_mg_build_coarse_op.  NULL = the
+                                     sweeps' result: in FP64, at even edges 10..32 and
+                                     enough sweeps, as a polynomial of the sweep map (equal
+                                     to rounding), else sweep by sweep.  WF_MG_COP_SWEEPS =
+                                     sweep by sweep always */
   void* mg_cop_part;              /* this case's scratch for it (N/2 elements) */
 } wf_case;
 
@@ -128,8 +134,14 @@ WF_API int wf_struct_sizes(int64_t* scalars, int64_t* casebytes);
 WF_API int wf_scalars_init(wf_scalars* sc, double dt0, double rrey, double ulid, void* stream);
 /* Tuning knob (no reference counterpart): how a many-sweep relax of an n^3
  * level (n <= 64) runs -- 0 one CTA, 1 cluster with a barrier per
- * half-sweep, 2 cluster with point-to-point halo pushes.  Process-wide;
- * set before graphs are built.  fp32 selects the mixed-precision table. */
+ * half-sweep, 2 cluster with point-to-point halo pushes, 3 the same with two
+ * halo planes and one exchange per sweep, 4 point-to-point with thinner
+ * slabs.  Setting one also makes the coarsest FP64 relax of that size run as
+ * these sweeps; with WF_COARSE_POLY added (the default state of every size)
+ * it is summed as their polynomial instead, where that applies (see mg_cop).
+ * Process-wide; set before graphs are built.  fp32 selects the
+ * mixed-precision table. */
+#define WF_COARSE_POLY 8
 WF_API int wf_set_coarse_strategy(int32_t n, int32_t fp32, int32_t strategy);
 /* Tuning knob (no reference counterpart): the launch shape of a kernel for
  * size n.  kind 0 = the convection pass (k_conv): a x b threads per CTA, a
@@ -170,7 +182,7 @@ WF_API int wf_mg_coarse_op_elems(const wf_case* c, int64_t* op_elems, int64_t* s
 WF_API int wf_mg_build_coarse_op(const wf_case* c, void* stream);
 /* The coarsest-level solve of a V-cycle (multigrid.py:301-322, coarsest
  * level: phi from zero, n_coarse sweeps) on an explicit FP64 pair of
- * (n_c+2)^3 doubles: through c->mg_cop when it is set, else as sweeps. */
+ * (n_c+2)^3 doubles, as a V-cycle of the case runs it (c->mg_cop). */
 WF_API int wf_mg_coarse_solve(const wf_case* c, double* phi, const double* rhs, void* stream);
 
 /* ---- initial state ---------------------------------------------------- */

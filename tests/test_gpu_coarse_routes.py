@@ -1,4 +1,6 @@
-"""The coarsest-level solve on its own is the one a V-cycle runs."""
+"""The coarsest-level solve on its own is the one a V-cycle runs; its forms -- the
+operator, the polynomial of the sweep map, literal sweeps -- can each be had and
+agree."""
 import ctypes
 
 import numpy as np
@@ -55,3 +57,92 @@ def test_coarse_solve_is_the_vcycles(nc):
     got = _coarse_solve(mg, c, lev1.rhs.numpy())
     assert np.abs(want).max() > 0
     np.testing.assert_array_equal(got, want)
+
+
+def _sweeps(nc, rhs, n_coarse):
+    """The relax a few sweeps at a time: neither polynomial nor operator."""
+    from warpflow import Multigrid, build_topology
+    cfg = make_cfg(nc, levels=1)
+    h = 1.0 / nc
+    one = Multigrid(cfg, build_topology(cfg), "cuda:0", *(h * x for x in HS))
+    one.levels[0].rhs.assign(rhs)
+    one.levels[0].phi.zero_()
+    for part in [12] * (n_coarse // 12) + [n_coarse % 12]:
+        one._relax(0, part)
+    return one.levels[0].phi.numpy()[1:-1, 1:-1, 1:-1]
+
+
+def _chosen(kind, nc):
+    """(case of a coarse solve of edge nc, undo): polynomial by default, literal
+    sweeps by the case, by the size's strategy."""
+    from warpflow import autotune
+    default = 0 if nc <= 16 else (2 if nc == 20 else 4)
+    autotune.set_strategy(nc, default, poly=kind != "strategy")
+    mg = _mg(nc, coarse="sweeps") if kind == "case" else _mg(nc)
+    mg.n_coarse = 300
+    return mg, mg.case() if kind == "case" else _no_operator(mg)
+
+
+@pytest.mark.parametrize("nc", [10, 14, 18, 22, 26, 30])
+def test_literal_sweeps_can_be_had(nc):
+    """`mg_coarse: sweeps` and a chosen strategy run the sweeps themselves: at
+    these edges the bits of a few sweeps at a time; the default does not."""
+    from warpflow import autotune
+    rhs = _rhs(nc, nc)
+    want = _sweeps(nc, rhs, 300)
+    try:
+        for kind, literal in (("case", True), ("strategy", True), ("default", False)):
+            got = _coarse_solve(*_chosen(kind, nc), rhs)
+            assert np.array_equal(got, want) == literal, kind
+            # a rounding per sweep
+            assert np.abs(got - want).max() <= 300 * 2.3e-16 * np.abs(want).max()
+    finally:
+        autotune.set_strategy(nc, 0 if nc <= 16 else 4, poly=True)
+
+
+@pytest.mark.parametrize("nc", EDGES)
+def test_operator_and_polynomial_match_literal_sweeps(nc):
+    """A whole V-cycle of every form against one whose coarsest level is swept."""
+    from warpflow import _abi, autotune
+    autotune.set_strategy(nc, 0 if nc <= 16 else (2 if nc == 20 else 4), poly=True)
+    out = {}
+    for name in ("sweeps", "polynomial", "operator"):
+        mg = _mg(nc, coarse="sweeps" if name == "sweeps" else "operator")
+        c = _no_operator(mg) if name == "polynomial" else mg.case()
+        lev = mg.levels[0]
+        lev.rhs.assign(np.random.default_rng(nc).standard_normal(lev.shape))
+        lev.phi.zero_()
+        _abi.call("wf_mg_vcycle", ctypes.byref(c), lev.phi.ptr, lev.rhs.ptr, mg._stream())
+        out[name] = lev.phi.numpy()[1:-1, 1:-1, 1:-1]
+    assert not np.array_equal(out["polynomial"], out["sweeps"])
+    for name in ("polynomial", "operator"):
+        assert np.abs(out[name] - out["sweeps"]).max() <= 1e-12 * np.abs(out["sweeps"]).max()
+
+
+def test_tuned_strategies_keep_the_polynomial(tmp_path):
+    """A tuned table, and one saved before tables said so, leave the polynomial
+    where it is faster; the sentinel is no operator to build into."""
+    from warpflow import _abi, autotune
+    rhs = _rhs(18, 3)
+    want = _coarse_solve(*_chosen("default", 18), rhs)
+    try:
+        table = autotune.tune(sizes=(14, 24), sweeps=300)
+        assert table[14]["poly"] and table[24]["poly"]
+        old = tmp_path / "old.json"
+        autotune.save({18: {"best": 4, "us": {"4": 1.0}}}, old)
+        autotune.load_and_apply(old)
+        mg = _mg(18)
+        np.testing.assert_array_equal(_coarse_solve(mg, _no_operator(mg), rhs), want)
+        off = tmp_path / "off.json"
+        autotune.save({18: {"best": 4, "us": {"4": 1.0}, "poly": False}}, off)
+        autotune.load_and_apply(off)
+        assert not np.array_equal(_coarse_solve(mg, _no_operator(mg), rhs), want)
+    finally:
+        for n in (14, 18, 24):
+            autotune.set_strategy(n, 0 if n <= 16 else 4, poly=True)
+            autotune.set_strategy(n, 0 if n <= 16 else 4, fp32=True)
+    c = _mg(24, coarse="sweeps").case()
+    with pytest.raises(RuntimeError):
+        _abi.call("wf_mg_build_coarse_op", ctypes.byref(c), None)
+    with pytest.raises(RuntimeError):
+        autotune.set_strategy(24, 5)

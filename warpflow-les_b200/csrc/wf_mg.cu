@@ -2200,7 +2200,8 @@ static bool g_strategy_init = false;
 
 static void strategy_defaults() {
   for (int f = 0; f < 2; ++f)
-    for (int n = 0; n <= 64; ++n) g_strategy[f][n] = n <= 16 ? 0 : (n == 20 ? 2 : 4);
+    for (int n = 0; n <= 64; ++n)
+      g_strategy[f][n] = (n <= 16 ? 0 : (n == 20 ? 2 : 4)) | WF_COARSE_POLY;
   g_strategy_init = true;
 }
 
@@ -2208,12 +2209,23 @@ static int coarse_strategy(int n, bool fp32) {
   const char* e = getenv("WF_COARSE");
   if (e && e[0] >= '0' && e[0] <= '4') return e[0] - '0';
   if (!g_strategy_init) strategy_defaults();
-  return (n >= 0 && n <= 64) ? g_strategy[fp32 ? 1 : 0][n] : 2;
+  return (n >= 0 && n <= 64) ? g_strategy[fp32 ? 1 : 0][n] & ~WF_COARSE_POLY : 2;
+}
+
+// whether an FP64 coarsest relax from zero may be summed as a polynomial: not
+// where a strategy was chosen for its sweeps
+static bool coarse_poly(int n) {
+  const char* e = getenv("WF_COARSE");
+  if (e && e[0] >= '0' && e[0] <= '4') return false;
+  if (!g_strategy_init) strategy_defaults();
+  return n >= 0 && n <= 64 && (g_strategy[0][n] & WF_COARSE_POLY);
 }
 
 int set_coarse_strategy(int n, int fp32, int strategy) {
-  if (n < 0 || n > 64 || strategy < 0 || strategy > 4)
-    return fail(WF_EINVAL, "wf_set_coarse_strategy: n in 0..64, strategy in 0..4");
+  const int sweeps = strategy & ~WF_COARSE_POLY;
+  if (n < 0 || n > 64 || sweeps < 0 || sweeps > 4)
+    return fail(WF_EINVAL, "wf_set_coarse_strategy: n in 0..64, strategy in 0..4, optionally | "
+                           "WF_COARSE_POLY");
   if (!g_strategy_init) strategy_defaults();
   g_strategy[fp32 ? 1 : 0][n] = strategy;
   return WF_OK;
@@ -3128,16 +3140,16 @@ static int launch_relax_smem(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
 // rhs_ready: the level's rhs is unchanged since its last relax, so a split
 // copy of it made then can be reused
 // zero: the level's phi is zero (a level after the restriction)
-// last: the coarsest level; first: the launch ahead made the first half-sweep
-// (only where relax_by_launches)
+// poly: the coarsest level of a case that lets its sweeps be summed; first: the
+// launch ahead made the first half-sweep (only where relax_by_launches)
 template <class T>
 static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = false,
-                 bool zero = false, bool last = false, bool first = false) {
+                 bool zero = false, bool poly = false, bool first = false) {
   if (nsweeps <= 0) return WF_OK;
   if (relax_by_launches(L, nsweeps)) return launch_sweeps(L, nsweeps, s, rhs_ready, first);
   {
     int rc = WF_OK;
-    if (zero && last && try_coarse_cheb(L, nsweeps, s, &rc)) return rc;
+    if (zero && poly && coarse_poly(L.n) && try_coarse_cheb(L, nsweeps, s, &rc)) return rc;
   }
   // a bucket launch serves many cases through their table: only kernels that
   // take one (the one-CTA column kernel, split and plain sweeps, the
@@ -3185,6 +3197,11 @@ static int relax(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_ready = 
   return launch_sweeps(L, nsweeps, s, rhs_ready, false);
 }
 
+// the case brings a coarse operator
+static bool has_cop(const wf_case& c) {
+  return c.mg_cop && c.mg_cop != WF_MG_COP_SWEEPS && c.mg_cop_part;
+}
+
 // a level the V-cycle keeps in the split layout: one that relax() would send
 // to relax_split for both smoothings
 template <class T>
@@ -3226,14 +3243,13 @@ static int vcycle(std::vector<Lvl<T>>& lv, const wf_case& c, cudaStream_t s,
       first = zero0;
       WF_TRY(split_in(lv[0], !rhs0_ready, s, zero0));
     }
-    if (l == L - 1 && L > 1 && c.mg_cop && c.mg_cop_part && c.n_coarse >= 2 &&
-        cop_size_ok(lv[l].n))
+    if (l == L - 1 && L > 1 && has_cop(c) && c.n_coarse >= 2 && cop_size_ok(lv[l].n))
       WF_TRY(apply_coarse_op<T>(lv[l], (const T*)c.mg_cop, (T*)c.mg_cop_part, s));
     else if (res[l])
       WF_TRY(split_sweeps(lv[l], c.n_pre, s, false, first));
     else
       WF_TRY(relax(lv[l], l < L - 1 ? c.n_pre : c.n_coarse, s, l == 0 && rhs0_ready,
-                   l > 0, l == L - 1, first));
+                   l > 0, l == L - 1 && c.mg_cop != WF_MG_COP_SWEEPS, first));
   }
   // the post-smoothing starts with colour 0, from the other colour alone: the
   // prolongation need not make the cells it overwrites
@@ -3476,7 +3492,8 @@ int coarse_op_elems(const wf_case& c, int64_t* op_elems, int64_t* scratch_elems)
 }
 
 int build_coarse_op_case(const wf_case& c, cudaStream_t s) {
-  if (!c.mg_cop) return fail(WF_EINVAL, "mg_cop is null");
+  if (!c.mg_cop || c.mg_cop == WF_MG_COP_SWEEPS)
+    return fail(WF_EINVAL, "mg_cop is null or WF_MG_COP_SWEEPS");
   WF_TRY(coarse_op_elems(c, nullptr, nullptr));
   const int l = c.nlev - 1;
   double a[3];
@@ -3600,7 +3617,7 @@ int mg_relax_pair(const wf_case& c, double* phi0, const double* rhs0, int nsweep
 
 // the coarsest-level solve of a V-cycle on an explicit (n_c+2)^3 pair: phi
 // from zero by the case's coarse operator when it has one, else n_coarse
-// sweeps
+// sweeps or their polynomial
 int mg_coarse_solve_pair(const wf_case& c, double* phi, const double* rhs, cudaStream_t s) {
   if (c.nlev < 2) return fail(WF_EINVAL, "coarse solve needs nlev >= 2");
   const int l = c.nlev - 1;
@@ -3621,9 +3638,9 @@ int mg_coarse_solve_pair(const wf_case& c, double* phi, const double* rhs, cudaS
   const long m = (long)L.n + 2;
   WF_CK(launch_k(k_zero<double>, mg_blocks(m * m * m), MG_TPB, 0, s, phi, m * m * m, -1));
   WF_CKL("k_zero");
-  if (c.mg_cop && c.mg_cop_part && !c.mg_fp32 && c.n_coarse >= 2 && cop_size_ok(L.n))
+  if (has_cop(c) && !c.mg_fp32 && c.n_coarse >= 2 && cop_size_ok(L.n))
     return apply_coarse_op<double>(L, (const double*)c.mg_cop, (double*)c.mg_cop_part, s);
-  return relax<double>(L, c.n_coarse, s, false, true, true);
+  return relax<double>(L, c.n_coarse, s, false, true, c.mg_cop != WF_MG_COP_SWEEPS);
 }
 
 int mg_refill_pair(const wf_case& c, double* phi0, cudaStream_t s) {

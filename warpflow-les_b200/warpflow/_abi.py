@@ -16,6 +16,9 @@ FIELD_NAMES = ("u", "v", "w", "p", "ustar", "vstar", "wstar", "uoo", "voo",
 
 ST_OK, ST_DT_COLLAPSE, ST_DIVERGED, ST_NOT_CONVERGED, ST_WAIT_TIMEOUT = range(5)
 
+MG_COP_SWEEPS = 1   # WF_MG_COP_SWEEPS: the coarsest relax sweep by sweep
+COARSE_POLY = 8     # WF_COARSE_POLY
+
 LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "libwfb200.so")
 
 

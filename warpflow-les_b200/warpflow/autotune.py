@@ -6,7 +6,9 @@ barrier per half-sweep; 2: a cluster with point-to-point halo pushes; 3: the
 same with two halo planes and one exchange per sweep; 4: point-to-point
 with thinner slabs, clusters of up to 16 CTAs) on a 300-sweep relax
 and installs the fastest through
-``wf_set_coarse_strategy``.
+``wf_set_coarse_strategy``.  A V-cycle's coarsest FP64 relax starts from zero
+and may run as a polynomial of the sweep map instead; the tuner times that solve
+both ways and leaves the polynomial on unless the sweeps are faster.
 
 ``tune_buckets`` makes the ensemble's choice per case size: it times an
 ensemble step of ``ncases`` equal-sized cases bucketed (every kernel launch
@@ -60,13 +62,33 @@ def _time_relax(mg, sweeps, reps=3):
     return a.elapsed_time(b) / reps * 1e3  # us
 
 
-def set_strategy(n, strategy, fp32=False):
-    _abi.call("wf_set_coarse_strategy", int(n), 1 if fp32 else 0, int(strategy))
+def set_strategy(n, strategy, fp32=False, poly=False):
+    """How a many-sweep relax of edge n runs.  Sweeps chosen here are what runs;
+    with `poly` (the library's default state) the coarsest FP64 relax of a
+    V-cycle is summed as their polynomial where that applies."""
+    _abi.call("wf_set_coarse_strategy", int(n), 1 if fp32 else 0,
+              int(strategy) | (_abi.COARSE_POLY if poly else 0))
+
+
+def _time_coarse(n, sweeps, device, reps=3):
+    """us of the coarsest solve of edge n without an operator, as installed."""
+    cfg = case_from_dict({"grid": {"nx": 2 * n, "ny": 2 * n, "nz": 2 * n},
+                          "numerics": {"mg_levels": 2}})
+    h = 0.5 / n
+    mg = Multigrid(cfg, build_topology(cfg), device, h, h, h, coarse="sweeps")
+    mg.n_coarse = sweeps
+    lev = mg.levels[1]
+    lev.rhs.assign(np.random.default_rng(n).standard_normal(lev.shape))
+    c = mg.case()
+    c.mg_cop = None
+    return _time_fn(lambda: _abi.call("wf_mg_coarse_solve", ctypes.byref(c), lev.phi.ptr,
+                                      lev.rhs.ptr, mg._stream()), reps)
 
 
 def tune(sizes=SIZES, sweeps=300, device="cuda:0"):
     """Time every applicable strategy for each size; install and return
-    {n: {"best": s, "us": {s: time}}}."""
+    {n: {"best": s, "us": {s: time}, "poly": p}}, p whether the coarsest FP64
+    relax stays a polynomial."""
     if os.environ.get("WF_COARSE"):
         raise RuntimeError("unset WF_COARSE to autotune (it forces one strategy)")
     out = {}
@@ -85,9 +107,15 @@ def tune(sizes=SIZES, sweeps=300, device="cuda:0"):
             lev.phi.zero_()
             times[s] = _time_relax(mg, sweeps)
         best = min(times, key=times.get)
-        set_strategy(n, best)
         set_strategy(n, best, fp32=True)
-        out[n] = {"best": best, "us": {str(k): round(v, 1) for k, v in times.items()}}
+        t = {}
+        for p in (False, True):
+            set_strategy(n, best, poly=p)
+            t[p] = _time_coarse(n, sweeps, device)
+        poly = t[True] <= 1.05 * t[False]   # the two are one route at most sizes
+        set_strategy(n, best, poly=poly)
+        out[n] = {"best": best, "us": {str(k): round(v, 1) for k, v in times.items()},
+                  "poly": poly}
     return out
 
 
@@ -266,7 +294,8 @@ def load_and_apply(path, fp32_buckets=True):
     sections = ("coarse", "buckets", "shapes")
     coarse = doc.get("coarse", {} if any(k in doc for k in sections) else doc)
     for n, rec in coarse.items():
-        set_strategy(int(n), rec["best"])
+        # tables that do not say: the best of the sweeps, the polynomial as it is
+        set_strategy(int(n), rec["best"], poly=rec.get("poly", True))
         set_strategy(int(n), rec["best"], fp32=True)
     for n, rec in doc.get("buckets", {}).items():
         set_bucket_cap(int(n), rec["cap"], fp32_buckets)

@@ -10,7 +10,8 @@ Two additions: ``numerics.mg_precision`` selects the multigrid arithmetic,
 an FP64 defect correction); ``numerics.mg_coarse`` selects how the coarsest
 level's n_coarse sweeps run, ``"operator"`` (default: the same linear map
 applied as one precomputed matrix-vector product, where the coarsest edge is
-4..24 in steps of 4) or ``"sweeps"``.
+4..24 in steps of 4, and in FP64 as a polynomial of the sweep map at the other
+even edges up to 32) or ``"sweeps"`` (sweep by sweep).
 """
 from __future__ import annotations
 

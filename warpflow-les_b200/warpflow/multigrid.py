@@ -32,6 +32,7 @@ process; each instance keeps its own partial-sum scratch.  Where the
 coarsest edge is not 4..24 in steps of 4, n_coarse < 2, or the operator
 would exceed ``COARSE_OP_MAX_BYTES``, the sweeps run: in FP64 at even edges
 10..32 as a polynomial of the sweep map, else one by one.
+``coarse="sweeps"`` runs them one by one at every edge.
 """
 from __future__ import annotations
 
@@ -212,6 +213,8 @@ class Multigrid:
             cop = self._coarse_op(c)
             if cop is not None:
                 c.mg_cop, c.mg_cop_part = cop[0].data_ptr(), cop[1].data_ptr()
+            elif self.coarse == "sweeps":
+                c.mg_cop = _abi.MG_COP_SWEEPS
         if su is not None:
             c.fld[_abi.FIELD_NAMES.index("su")] = su.ptr
         if pp is not None:
@@ -235,7 +238,7 @@ class Multigrid:
         Multigrid uses one, else n_coarse sweeps."""
         lev = self.levels[-1]
         c = self.case()
-        if c.mg_fp32:   # the FP32 operator serves FP32 levels only
+        if c.mg_fp32 and c.mg_cop_part:   # the FP32 operator serves FP32 levels only
             c.mg_cop = c.mg_cop_part = None
         _abi.call("wf_mg_coarse_solve", ctypes.byref(c), lev.phi.ptr, lev.rhs.ptr,
                   self._stream())
