@@ -146,3 +146,51 @@ def test_tuned_strategies_keep_the_polynomial(tmp_path):
         _abi.call("wf_mg_build_coarse_op", ctypes.byref(c), None)
     with pytest.raises(RuntimeError):
         autotune.set_strategy(24, 5)
+
+
+def _exact_sweeps(nc, rhs, n_coarse):
+    """The sweeps in extended precision; the diagonal is the kernels', summed in
+    double (its rounding is the problem's, not the sweeps')."""
+    LD = np.longdouble
+    n = nc
+    h = 1.0 / (2 * nc)
+    a = [1.0 / ((2 * (h * x)) * (2 * (h * x))) for x in HS]
+    at = np.indices((n,) * 3)
+    co = []
+    ap = np.zeros((n,) * 3)
+    for ax in range(3):
+        co += [np.where(at[ax] > 0, a[ax], 0.0), np.where(at[ax] < n - 1, a[ax], 0.0)]
+        ap = ap + co[-2] + co[-1]
+    ap = -ap.astype(LD)
+    phi = np.zeros((n + 2,) * 3, LD)
+    r = rhs[1:-1, 1:-1, 1:-1].astype(LD)
+    mid = slice(1, -1)
+    nb = [(slice(0, -2), mid, mid), (slice(2, None), mid, mid), (mid, slice(0, -2), mid),
+          (mid, slice(2, None), mid), (mid, mid, slice(0, -2)), (mid, mid, slice(2, None))]
+    core = phi[mid, mid, mid]
+    masks = [(at.sum(0) + c) % 2 == 1 for c in (0, 1)]
+    for _ in range(n_coarse):
+        for m in masks:
+            x = (r - sum(co[q] * phi[nb[q]] for q in range(6))) / ap
+            core[m] = x[m]
+    return core.copy()
+
+
+# Mean over 12 right-hand sides.  One error varies by about a third with the
+# right-hand side, so each mean is known to a tenth and the ratio of two to 15 %;
+# 1.25 is that and a little.  A tail of 16 sweeps gave 1.5 and 1.8.
+def test_polynomial_is_as_close_as_the_sweeps():
+    err = []
+    for nc in (10, 14, 18, 22):
+        mg, c = _chosen("default", nc)
+        for seed in range(3):
+            rhs = _rhs(nc, 10 * nc + seed)
+            ref = _exact_sweeps(nc, rhs, 300)
+            row = []
+            for got in (_coarse_solve(mg, c, rhs), _sweeps(nc, rhs, 300)):
+                e = (got - ref).astype(float)
+                row.append((np.abs(e).max() / float(np.abs(ref).max()),
+                            float(np.sqrt((e ** 2).mean() / (ref ** 2).mean()))))
+            err.append(row)
+    poly, sweeps = np.array(err).mean(0)
+    assert (poly <= 1.25 * sweeps).all(), (poly, sweeps)

@@ -1244,23 +1244,31 @@ static int try_coarse_p2p(const Lvl<T>& L, int nsweeps, cudaStream_t s, int* rc)
 // of about 5.8 sqrt(m) terms to the last bit of an FP64 result (degree 97 in
 // place of 283 sweeps), summed by Clenshaw's recurrence (C. W. Clenshaw, "A note
 // on the summation of Chebyshev series", MTAC 9, 1955).  A term costs one sweep
-// with a zero rhs.  The last CHEB_TAIL + 1 sweeps run as such: they damp the
-// recurrence's rounding errors, and the result stays as close to exact
-// arithmetic as the sweeps' (about 1e-15 of its size).
-// us per 300-sweep relax, FP64, sweeps / polynomial: 10^3 279 / 140, 18^3 393 /
-// 183, 24^3 380 / 206, 32^3 466 / 270.
+// with a zero rhs.  The last tail + 1 sweeps run as such: they damp the
+// recurrence's rounding errors, and tail is as long as it takes for the result to
+// be no further from exact arithmetic than the sweeps it stands for.  Off the
+// multiples of four those are sweeps with the exact quotient: mean of the largest
+// and of the r.m.s. error over 144 right-hand sides of edges 10..30, 300 sweeps,
+// relative to the sweeps': tail 16 1.53 / 1.77, 32 1.07 / 1.09, 48 1.00 / 0.99, 64
+// 0.96 / 0.90 (450 sweeps 0.89 / 0.83, 200 sweeps 0.99 / 0.95).  On the multiples
+// of four they multiply by the diagonal's reciprocal, which costs them more than
+// any tail: 16 gives 0.17 / 0.09.
+// us per 300-sweep relax in a graph, FP64, sweeps / polynomial: 10^3 269 / 166, 14^3
+// 337 / 199, 18^3 385 / 219, 22^3 400 / 242, 24^3 390 / 193, 26^3 460 / 266, 30^3
+// 577 / 331, 32^3 545 / 246.
 constexpr int CHEB_MAX = 128;
-constexpr int CHEB_TAIL = 16;
+static constexpr int cheb_tail(int n) { return n % 4 ? 64 : 16; }
 struct ChebCoef {
   double c[CHEB_MAX];
   int deg;
+  int tail;
 };
 
 // coefficients of sum_{s<m} ((1 + t) / 2)^s, cut where the rest is below an ulp
 // of the sum (m); deg < 0 when CHEB_MAX terms do not reach that.  The row of
 // 4^-s C(2s, s-k) is a random walk's distribution: positive terms only.
-static const ChebCoef& cheb_coef(int m) {
-  static thread_local ChebCoef last{{}, -2};
+static ChebCoef& cheb_coef(int m) {
+  static thread_local ChebCoef last{{}, -2, 0};
   static thread_local int last_m = -1;
   if (last_m == m) return last;
   std::vector<double> p(CHEB_MAX + 2, 0.0), q(CHEB_MAX + 2, 0.0), sum(CHEB_MAX + 2, 0.0);
@@ -1397,8 +1405,8 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     mbar_arrive_expect_tx(mb[1], tx);
   }
   cl.sync();  // barriers armed and planes zeroed in every CTA
-  // the first sweep, deg terms, CHEB_TAIL + 1 sweeps
-  const int nh = 2 * (1 + C.deg + CHEB_TAIL + 1);
+  // the first sweep, deg terms, tail + 1 sweeps
+  const int nh = 2 * (1 + C.deg + C.tail + 1);
   bool bailed = false;
   for (int t = 0; t < nh; ++t) {
     if (t > 0) {
@@ -1504,9 +1512,12 @@ static int launch_coarse_cheb(const Lvl<double>& L, const ChebCoef& C, cudaStrea
 // serves it, in a bucket too (a case computes the same bits alone and in one):
 // where it saves at least a third of the sweeps
 static int try_coarse_cheb(const Lvl<double>& L, int nsweeps, cudaStream_t s, int* rc) {
-  if (nsweeps < 64) return 0;
-  const ChebCoef& C = cheb_coef(nsweeps - 1 - CHEB_TAIL);
-  if (C.deg < 1 || 3 * (C.deg + 2 + CHEB_TAIL) > 2 * nsweeps) return 0;
+  const int tail = cheb_tail(L.n);
+  // more than about 490 sweeps before the tail do not fit CHEB_MAX terms
+  if (nsweeps < 64 || nsweeps > 512 + tail) return 0;
+  ChebCoef& C = cheb_coef(nsweeps - 1 - tail);
+  C.tail = tail;
+  if (C.deg < 1 || 3 * (C.deg + 2 + tail) > 2 * nsweeps) return 0;
   switch (L.n) {
     case 10: *rc = launch_coarse_cheb<10, 1>(L, C, s); return 1;
     case 12: *rc = launch_coarse_cheb<12, 2>(L, C, s); return 1;
