@@ -1023,14 +1023,12 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
   const int rank = (int)cl.block_rank();
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ __align__(8) unsigned long long mbar[2];
-  __shared__ int s_bail;
   T* sp = reinterpret_cast<T*>(smraw);
   const int tid = threadIdx.x;
   const uint32_t mb[2] = {smem_u32(&mbar[0]), smem_u32(&mbar[1])};
   if (tid == 0) {
     mbar_init(mb[0], 1);
     mbar_init(mb[1], 1);
-    s_bail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int t = tid; t < 2 * NC * PL; t += blockDim.x) sp[t] = T(0);
@@ -1094,17 +1092,18 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
   const int nh = 2 * nsweeps;
   bool bailed = false;
   for (int t = 0; t < nh; ++t) {
+    bool ok = true;
     if (t > 0) {
       // halo values of the colour read now were produced at t-1
       const int c = (t - 1) & 1;
       const uint32_t par = (uint32_t)(((t - 1) >> 1) & 1);
-      bool ok = false;
+      ok = false;
       for (int it = 0; it < MBAR_WAIT_TRIES && !ok; ++it) ok = mbar_try_wait(mb[c], par, wmode);
-      if (!ok) s_bail = 1;
       if (tid == 0 && t + 1 < nh) mbar_arrive_expect_tx(mb[c], tx);
     }
-    __syncthreads();  // local values of t-1 visible; bail decision uniform
-    if (s_bail) {
+    // local values of t-1 visible; every thread gets the same answer, so that all
+    // of them leave the loop at the same barrier
+    if (__syncthreads_or(!ok)) {
       bailed = true;
       break;
     }
@@ -1137,10 +1136,10 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     const uint32_t par = (uint32_t)(((nh - 1) >> 1) & 1);
     bool ok = false;
     for (int it = 0; it < MBAR_WAIT_TRIES && !ok; ++it) ok = mbar_try_wait(mb[c], par, wmode);
-    if (!ok) s_bail = 1;
+    bailed = !ok;
   }
-  __syncthreads();
-  if (s_bail && tid == 0 && L.err) atomicExch(L.err, (int)WF_ST_WAIT_TIMEOUT);
+  bailed = __syncthreads_or(bailed);
+  if (bailed && tid == 0 && L.err) atomicExch(L.err, (int)WF_ST_WAIT_TIMEOUT);
   cl.sync();
   if (!active) return;
 #pragma unroll
@@ -1346,7 +1345,6 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
   const int rank = (int)cl.block_rank();
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ __align__(8) unsigned long long mbar[2];
-  __shared__ int s_bail;
   T* sp = reinterpret_cast<T*>(smraw);
   const int tid = threadIdx.x;
   const uint32_t mb[2] = {smem_u32(&mbar[0]), smem_u32(&mbar[1])};
@@ -1355,7 +1353,6 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
   if (tid == 0) {
     mbar_init(mb[0], 1);
     mbar_init(mb[1], 1);
-    s_bail = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int t = tid; t < 2 * NC * PL; t += blockDim.x) sp[t] = T(0);
@@ -1409,16 +1406,15 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
   const int nh = 2 * (1 + C.deg + C.tail + 1);
   bool bailed = false;
   for (int t = 0; t < nh; ++t) {
+    bool ok = true;
     if (t > 0) {
       const int c = (t - 1) & 1;
       const uint32_t par = (uint32_t)(((t - 1) >> 1) & 1);
-      bool ok = false;
+      ok = false;
       for (int it = 0; it < MBAR_WAIT_TRIES && !ok; ++it) ok = mbar_try_wait(mb[c], par, wmode);
-      if (!ok) s_bail = 1;
       if (tid == 0 && t + 1 < nh) mbar_arrive_expect_tx(mb[c], tx);
     }
-    __syncthreads();
-    if (s_bail) {
+    if (__syncthreads_or(!ok)) {
       bailed = true;
       break;
     }
@@ -1466,10 +1462,10 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     const uint32_t par = (uint32_t)(((nh - 1) >> 1) & 1);
     bool ok = false;
     for (int it = 0; it < MBAR_WAIT_TRIES && !ok; ++it) ok = mbar_try_wait(mb[c], par, wmode);
-    if (!ok) s_bail = 1;
+    bailed = !ok;
   }
-  __syncthreads();
-  if (s_bail && tid == 0 && L.err) atomicExch(L.err, (int)WF_ST_WAIT_TIMEOUT);
+  bailed = __syncthreads_or(bailed);
+  if (bailed && tid == 0 && L.err) atomicExch(L.err, (int)WF_ST_WAIT_TIMEOUT);
   cl.sync();
   if (!active) return;
 #pragma unroll
