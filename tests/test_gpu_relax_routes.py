@@ -186,3 +186,20 @@ def test_odd_coarsest_level_from_the_host_and_in_a_graph():
     assert counts[0] < 300 and counts[1] - counts[0] == 4 * 599
     for a, b in zip(*fields):
         np.testing.assert_array_equal(a, b)
+
+
+def test_bucket_keeps_one_cta_for_a_small_coarsest_level():
+    """The 14^3 coarsest level of a mixed bucket: one launch for its 300 sweeps,
+    and the fields of the cases alone (which sweep in a cluster)."""
+    from warpflow import FlowSolver, build_topology
+    from warpflow.ensemble import Ensemble, cavity_case
+    cfgs = [cavity_case(56, re, 1.0, precision="mixed") for re in (200.0, 900.0)]
+    ens = Ensemble(cfgs, nstreams=1, buckets=True)
+    assert ens.layout()[1][0][2] < 600          # launches of the multigrid part
+    alone = [FlowSolver(c, build_topology(c), "cuda:0") for c in cfgs]
+    for _ in range(2):
+        assert ens.step() == [s.step() for s in alone]
+    for sol, ref in zip(ens.solvers, alone):
+        for name in ("u", "v", "w", "p"):
+            np.testing.assert_array_equal(sol.f[name].numpy(), ref.f[name].numpy())
+    ens.close()

@@ -3126,9 +3126,12 @@ static bool capturing(cudaStream_t s) {
 // 14.  From the host one CTA is up to 15, and to 17 for few sweeps: us for 12 / 40 /
 // 300 sweeps, one CTA, launches: 11^3 44 / 115 / 746, 101 / 297 / 1475, 13^3 56 / 145
 // / 972, 103 / 212 / 1463, 15^3 69 / 183 / 1235, 88 / 241 / 1695, 17^3 88 / 246 /
-// 1694, 99 / 279 / 1470.
+// 1694, 99 / 279 / 1470.  A bucket's launches cost as much in a graph (they come
+// one after the other and read the case table first): six mixed 56^3 cases, 14^3
+// coarsest, 5.73 ms a step with one CTA, 6.52 with launches.
 static bool one_cta(int n, int nsweeps, cudaStream_t s) {
-  return n <= 10 || (n <= (nsweeps <= 100 ? 17 : 15) && !capturing(s));
+  return n <= 10 ||
+         (n <= (nsweeps <= 100 ? 17 : 15) && (batch_ctx().tab || !capturing(s)));
 }
 
 template <class T>
