@@ -169,13 +169,13 @@ def test_one_sweep_at_a_time_equals_all(n):
 
 
 def test_odd_coarsest_level_from_the_host_and_in_a_graph():
-    """The 300 sweeps of an 11^3 coarsest level: one launch each when the host
+    """The 300 sweeps of a 13^3 coarsest level: one launch each when the host
     issues them, 600 in a graph, where a launch costs less; the same fields."""
     import ctypes
     from warpflow import FlowSolver, _abi, build_topology
     counts, fields = [], []
     for mode in ("host", "graph"):
-        sol = FlowSolver(make_cfg(44), build_topology(make_cfg(44)), "cuda:0", step_mode=mode)
+        sol = FlowSolver(make_cfg(52), build_topology(make_cfg(52)), "cuda:0", step_mode=mode)
         for _ in range(2):
             sol.step()
         c = (ctypes.c_int32 * 4)()

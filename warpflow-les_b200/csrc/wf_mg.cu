@@ -3121,16 +3121,17 @@ static bool capturing(cudaStream_t s) {
 
 // Whether one CTA sweeps the level in shared memory (k_relax_smem) rather than a
 // launch per half-sweep (the same bits).  A launch costs 1.1 us in a graph and
-// 2.5 us from the host.  In a graph one CTA is up to 10: us for 6 sweeps, one
+// 2.5 us from the host.  In a graph one CTA is up to 11: us for 6 sweeps, one
 // CTA / launches: 10^3 11.5 / 15.1, 11^3 18.1 / 15.1, 14^3 25.2 / 13.6, 22^3 78 /
-// 14.  From the host one CTA is up to 15, and to 17 for few sweeps: us for 12 / 40 /
+// 14; for 300, 11^3 735 / 677, but 30 cases of 44^3 side by side take 15.7 ms a step
+// with one CTA and 19.2 with launches.  From the host one CTA is up to 15, and to 17 for few sweeps: us for 12 / 40 /
 // 300 sweeps, one CTA, launches: 11^3 44 / 115 / 746, 101 / 297 / 1475, 13^3 56 / 145
 // / 972, 103 / 212 / 1463, 15^3 69 / 183 / 1235, 88 / 241 / 1695, 17^3 88 / 246 /
 // 1694, 99 / 279 / 1470.  A bucket's launches cost as much in a graph (they come
 // one after the other and read the case table first): six mixed 56^3 cases, 14^3
 // coarsest, 5.73 ms a step with one CTA, 6.52 with launches.
 static bool one_cta(int n, int nsweeps, cudaStream_t s) {
-  return n <= 10 ||
+  return n <= 11 ||
          (n <= (nsweeps <= 100 ? 17 : 15) && (batch_ctx().tab || !capturing(s)));
 }
 
