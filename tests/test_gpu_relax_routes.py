@@ -203,3 +203,32 @@ def test_bucket_keeps_one_cta_for_a_small_coarsest_level():
         for name in ("u", "v", "w", "p"):
             np.testing.assert_array_equal(sol.f[name].numpy(), ref.f[name].numpy())
     ens.close()
+
+
+def test_long_coarse_relaxes_leave_the_chip_to_other_cases():
+    """Six cases with an 11^3 coarsest level side by side: their long one-CTA
+    relaxes run beside one another and beside the other kernels, so a step of
+    all takes little longer than a step of one (1.1 times; 1.4 when the kernels
+    behind a relax held SMs while it ran)."""
+    import torch
+    from warpflow.ensemble import Ensemble, cavity_case
+
+    def step_ms(ens):
+        for _ in range(3):
+            ens.launch()
+        best = 1e9
+        for _ in range(5):
+            a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+            a.record()
+            ens.launch()
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        return best
+
+    cfgs = [cavity_case(44, 200.0 + 50.0 * q, 1.0, precision="fp64") for q in range(6)]
+    one = Ensemble(cfgs[:1], nstreams=1, buckets=False)
+    six = Ensemble(cfgs, nstreams=1, buckets=False)
+    assert step_ms(six) < 1.25 * step_ms(one)
+    one.close()
+    six.close()

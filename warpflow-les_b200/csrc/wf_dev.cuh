@@ -7,10 +7,10 @@
 
 namespace wf {
 
-// Programmatic dependent launch: every kernel of this library starts by
-// allowing its successor to begin launching, then waits until its
-// predecessor has completed and its memory is visible.  Without the launch
-// attribute both instructions are no-ops.
+// Programmatic dependent launch: a kernel allows its successor to begin
+// launching and waits until its predecessor has completed and its memory is
+// visible.  Without the launch attribute both instructions are no-ops.  The
+// kernels of wf_ops.cu start with both, in this order.
 //
 // The wait orders a kernel's global loads only if the compiler cannot move
 // them above it.  It is an asm statement with a memory clobber, but a load
@@ -30,9 +30,23 @@ __device__ __forceinline__ void pdl_entry() {
 // ahead of its wait runs when every kernel before its predecessor has
 // completed.  Data those wrote may therefore be read ahead of the wait
 // (__ldcg: past the L1, which may hold lines of an earlier pass).
-__device__ __forceinline__ void pdl_chain() {
+//
+// This is a contract between a kernel and the one launched ahead of it: a kernel
+// that reads varying data before pdl_wait must follow one that calls pdl_wait
+// before pdl_trigger (every kernel of the multigrid and the fills), not one that
+// starts with pdl_entry.  k_rbgs, k_rbgs_split, k_rbgs_flat, k_restrict and
+// k_coarse_cols do so only when their `pre` argument says that the data was
+// complete before the launch ahead, k_prolong and k_prolong8 always (they follow
+// the coarse relax); k_fill_one, k_cop_vg and k_cop_out read constants only.
+__device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_trigger() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void pdl_chain() {
+  pdl_wait();
+  pdl_trigger();
 }
 
 // ---- bucket batching (see Batch in wf_internal.h) -------------------------

@@ -505,13 +505,20 @@ __global__ void __launch_bounds__(MG_TPB) k_prolong8(const Lvl<T> C0, Lvl<T> F0,
   }
 }
 
+// A relax of many sweeps lets its successor launch only when the sweeps are done:
+// the successor's CTAs would hold SMs through all of them, which branches beside
+// this one could use.  ms a step of 6 and 13 cases side by side, early / late: 44^3
+// FP64 4.77 / 3.75 and 8.71 / 7.48, 72^3 mixed 3.63 / 2.99 and 7.66 / 6.25; one case
+// is as fast either way.
+constexpr int MANY_SWEEPS = 12;
+
 // ---- a whole relax() of a small level inside one CTA's shared memory ------
 // phi and rhs of the real cells live in shared memory ([i][j][k]); the
 // ring is not needed there because every ring term has a zero coefficient.
 // After the last sweep the interior and the face rings go back to global.
-template <class T>
+template <class T, bool MANY>
 __global__ void __launch_bounds__(1024) k_relax_smem(Lvl<T> L0, int nsweeps, const Batch bt) {
-  pdl_chain();
+  MANY ? pdl_wait() : pdl_chain();
   if (bt_skip(bt)) return;
   const Lvl<T> L = rebase(L0, bt);
   extern __shared__ __align__(16) unsigned char smraw[];
@@ -553,6 +560,7 @@ __global__ void __launch_bounds__(1024) k_relax_smem(Lvl<T> L0, int nsweeps, con
       __syncthreads();
     }
   }
+  if (MANY) pdl_trigger();
   for (int t = threadIdx.x; t < n3; t += blockDim.x) {
     const int k = t % n, j = (t / n) % n, i = t / (n * n);
     const long c = lid(L, i + 1, j + 1, k + 1);
@@ -633,15 +641,16 @@ struct CoarseShape {
 // With unit_out set, CTA b relaxes rhs = e_u from phi = 0, u the b-th cell
 // of even i+j+k in (i, j, k) order (cell index 2b or 2b+1), and writes the
 // even-parity cells of the result as row b of unit_out (position = cell
-// index / 2): the rows of the coarse-level operator.
-template <class T, int NC, bool RHS_SMEM>
+// index / 2): the rows of the coarse-level operator.  MANY: more than MANY_SWEEPS
+// sweeps.
+template <class T, int NC, bool RHS_SMEM, bool MANY>
 __global__ void __launch_bounds__(CoarseShape<NC>::THREADS) k_coarse_cols(Lvl<T> L0,
                                                                            int nsweeps, int pre,
                                                                            int zero, T* unit_out,
                                                                            const int* unit_ids,
                                                                            const Batch bt) {
   if (bt.tab) {
-    pdl_chain();
+    MANY ? pdl_wait() : pdl_chain();
     if (bt_skip(bt)) return;
     pre = 0;
   }
@@ -690,7 +699,7 @@ __global__ void __launch_bounds__(CoarseShape<NC>::THREADS) k_coarse_cols(Lvl<T>
   // b = unit_ids[blockIdx.x] (or blockIdx.x)
   const int ub = unit_ids ? unit_ids[blockIdx.x] : (int)blockIdx.x;
   const int unit = 2 * ub + (((2 * ub / NC) / NC + (2 * ub / NC) % NC) & 1);
-  if (!bt.tab) pdl_chain();
+  if (!bt.tab) MANY ? pdl_wait() : pdl_chain();
   if (unit_out) {
 #pragma unroll
     for (int k = 0; k < NC; ++k) {
@@ -750,6 +759,7 @@ __global__ void __launch_bounds__(CoarseShape<NC>::THREADS) k_coarse_cols(Lvl<T>
       __syncthreads();
     }
   }
+  if (MANY) pdl_trigger();
   if (unit_out) {
     if (!active) return;
     T* row = unit_out + (long)blockIdx.x * (NC * NC * NC / 2) + ((i * NC + j) * NC >> 1);
@@ -777,11 +787,12 @@ static int launch_coarse(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool pre,
                          T* unit_out = nullptr, const int* unit_ids = nullptr, int nunits = 0) {
   const size_t lvl = (size_t)2 * NC * CoarseShape<NC>::PLANE * sizeof(T);
   const size_t sb = RHS_SMEM || !unit_out ? 2 * lvl : lvl;
-  WF_CK(cudaFuncSetAttribute(k_coarse_cols<T, NC, RHS_SMEM>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * lvl)));
+  auto kern = nsweeps > MANY_SWEEPS ? k_coarse_cols<T, NC, RHS_SMEM, true>
+                                    : k_coarse_cols<T, NC, RHS_SMEM, false>;
+  WF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * lvl)));
   const int nb = unit_out ? (unit_ids ? nunits : NC * NC * NC / 2) : 1;
-  WF_CK(launch_chain(k_coarse_cols<T, NC, RHS_SMEM>, nb, CoarseShape<NC>::THREADS, sb, s, L,
-                     nsweeps, pre ? 1 : 0, zero ? 1 : 0, unit_out, unit_ids));
+  WF_CK(launch_chain(kern, nb, CoarseShape<NC>::THREADS, sb, s, L, nsweeps, pre ? 1 : 0,
+                     zero ? 1 : 0, unit_out, unit_ids));
   WF_CKL("k_coarse_cols");
   return WF_OK;
 }
@@ -822,7 +833,7 @@ struct ClusterShape {
 template <class T, int NC, int NCL>
 __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     k_coarse_cluster(Lvl<T> L, int nsweeps) {
-  pdl_chain();
+  pdl_wait();
   using S = ClusterShape<NC, NCL>;
   constexpr int H = S::H, HALF = S::HALF, GROUP = S::GROUP, PL = S::PL, C = S::C;
   namespace cg = cooperative_groups;
@@ -904,6 +915,7 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
       cl.sync();
     }
   }
+  pdl_trigger();
   if (!active) return;
 #pragma unroll
   for (int k = 0; k < NC; ++k) {
@@ -1015,7 +1027,7 @@ constexpr int MBAR_WAIT_TRIES = 1 << 22;
 template <class T, int NC, int NCL, bool EXACT>
 __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     k_coarse_p2p(Lvl<T> L, int nsweeps, int wmode) {
-  pdl_chain();
+  pdl_wait();
   using S = ClusterShape<NC, NCL>;
   constexpr int H = S::H, HALF = S::HALF, GROUP = S::GROUP, PL = S::PL, C = S::C;
   namespace cg = cooperative_groups;
@@ -1138,6 +1150,7 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     for (int it = 0; it < MBAR_WAIT_TRIES && !ok; ++it) ok = mbar_try_wait(mb[c], par, wmode);
     bailed = !ok;
   }
+  pdl_trigger();
   bailed = __syncthreads_or(bailed);
   if (bailed && tid == 0 && L.err) atomicExch(L.err, (int)WF_ST_WAIT_TIMEOUT);
   cl.sync();
@@ -1334,7 +1347,7 @@ __device__ __forceinline__ void cheb_cols(const double* __restrict__ oth, double
 template <int NC, int NCL>
 __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     k_coarse_cheb(Lvl<double> L0, const __grid_constant__ ChebCoef C, int wmode, const Batch bt) {
-  pdl_chain();
+  pdl_wait();
   if (bt_skip(bt)) return;   // the case's whole cluster
   const Lvl<double> L = rebase(L0, bt);
   using T = double;
@@ -1464,6 +1477,7 @@ __global__ void __launch_bounds__(ClusterShape<NC, NCL>::THREADS)
     for (int it = 0; it < MBAR_WAIT_TRIES && !ok; ++it) ok = mbar_try_wait(mb[c], par, wmode);
     bailed = !ok;
   }
+  pdl_trigger();
   bailed = __syncthreads_or(bailed);
   if (bailed && tid == 0 && L.err) atomicExch(L.err, (int)WF_ST_WAIT_TIMEOUT);
   cl.sync();
@@ -1584,7 +1598,7 @@ struct TbShape {
 template <class T, int NC, int NCL>
 __global__ void __launch_bounds__(TbShape<NC, NCL>::THREADS)
     k_coarse_tb(Lvl<T> L, int nsweeps, int wmode) {
-  pdl_chain();
+  pdl_wait();
   using S = TbShape<NC, NCL>;
   constexpr int H = S::H, HALF = S::HALF, GROUP = S::GROUP, PL = S::PL, C = S::C;
   constexpr int SIDE = S::SIDE;
@@ -1727,6 +1741,7 @@ __global__ void __launch_bounds__(TbShape<NC, NCL>::THREADS)
     __syncthreads();  // this sweep's reads of the halo planes are done
   }
   __syncthreads();
+  pdl_trigger();
   if (s_bail && tid == 0 && L.err) atomicExch(L.err, (int)WF_ST_WAIT_TIMEOUT);
   cl.sync();
   if (!do_black) return;
@@ -3140,10 +3155,10 @@ static int launch_relax_smem(const Lvl<T>& L, int nsweeps, cudaStream_t s) {
   const int n3 = L.n * L.n * L.n;
   const int tpb = std::min(1024, std::max(32, (n3 / 2 + 31) / 32 * 32));
   const size_t sb = 2 * (size_t)n3 * sizeof(T);
+  auto kern = nsweeps > MANY_SWEEPS ? k_relax_smem<T, true> : k_relax_smem<T, false>;
   if (sb > 48 * 1024)
-    WF_CK(cudaFuncSetAttribute(k_relax_smem<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)sb));
-  WF_CK(launch_chain(k_relax_smem<T>, 1, tpb, sb, s, L, nsweeps));
+    WF_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sb));
+  WF_CK(launch_chain(kern, 1, tpb, sb, s, L, nsweeps));
   WF_CKL("k_relax_smem");
   return WF_OK;
 }
