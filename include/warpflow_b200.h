@@ -146,10 +146,16 @@ WF_API int wf_set_coarse_strategy(int32_t n, int32_t fp32, int32_t strategy);
 /* Tuning knob (no reference counterpart): the launch shape of a kernel for
  * size n.  kind 0 = the convection pass (k_conv): a x b threads per CTA, a
  * along k (a power of two), b along j, a*b a multiple of 32 and <= 256,
- * and c consecutive planes i per thread (1..16); default 32 x 8 x 1.
- * kind 1 = the split red-black half-sweep of an n^3 level (k_rbgs_split):
- * a = cells per thread (1, 2, 4), b = rows per CTA (1, 2, 4, 8), c = 1;
- * default 2 x 8 x 1.  a = b = c = 0 restores the default.  Results do not
+ * and c consecutive planes i per thread (1..16); default 32 x 8 x 1 below
+ * 64, 32 x 4 x 2, and 32 x 4 x 4 from 192.
+ * kind 1 = the split red-black half-sweep of an n^3 level by rows
+ * (k_rbgs_split): a = cells per thread (1, 2, 4, 8), b = rows per CTA (1, 2,
+ * 4, 8), c = 1; default 4 x 8 below 100, 2 x 8, and 4 x 2 from 192.  By
+ * default only sizes from 104 that are below 144 or no multiple of 4 run by
+ * rows; below 104 and from 144 the half-sweep has other forms, which are faster
+ * there.  Setting a shape selects the rows form for FP64 levels of that size;
+ * FP32 levels keep their form and use the shape where that is rows.
+ * a = b = c = 0 restores the default.  Results do not
  * depend on the shape (each cell's arithmetic is the same).  Process-wide;
  * read when a launch is issued, so set it before steppers are built.
  * wf_launch_shape reads the shape in force. */

@@ -2610,8 +2610,8 @@ static int split_in(const Lvl<T>& L, bool with_rhs, cudaStream_t s, bool first =
 //    128^3 4.4 / 4.6, 160^3 10.4 / 7.2, 192^3 20.0 / 10.6, 256^3 35.0 / 24.2,
 //    320^3 106 / 47.  From 176 every second half-sweep runs its planes backward
 //    (what the one before touched last is still in L2: 256^3 FP64 41.5 -> 40.0).
-//  - Otherwise, and for a shape set for the level (wf_set_launch_shape), the
-//    rows of k_rbgs_split.
+//  - Otherwise, and in FP64 for a shape set for the level (wf_set_launch_shape,
+//    chosen by FP64 timings), the rows of k_rbgs_split.
 // rhs_ready: the split rhs was complete before the launch ahead of the first one;
 // first: the launch ahead made the first half-sweep (first_value)
 template <class T>
@@ -2621,7 +2621,7 @@ static int split_sweeps(const Lvl<T>& L, int nsweeps, cudaStream_t s, bool rhs_r
   T* sp = split_phi(L.tmp);
   const T* sr = split_rhs(L.tmp, n);
   const ApRecip<T> rt = ap_recip(L);
-  const bool set = launch_shape_set(SHAPE_SPLIT, n);
+  const bool set = sizeof(T) == 8 && launch_shape_set(SHAPE_SPLIT, n);
   const bool flat = n < FLAT_MAX_N && !set;
   const BatchCtx& bc = batch_ctx();
   const uintptr_t at = bc.tab ? bc.tmp_bits[L.role & 15] : (uintptr_t)L.tmp;   // every case's

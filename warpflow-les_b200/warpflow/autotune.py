@@ -17,11 +17,13 @@ faster through ``wf_set_bucket_cap``.
 
 ``tune_shapes`` chooses launch shapes per grid size: the CTA of the
 convection pass (``k_conv``: threads along k and j) and the cells per
-thread and rows per CTA of the split red-black half-sweep
-(``k_rbgs_split``).  Each candidate is timed on the kernel alone, its
+thread and rows per CTA of the split red-black half-sweep by rows
+(``k_rbgs_split``), against the form the library takes by itself, which at
+most sizes is another one (cells numbered flat, pairs marching through
+planes).  Each candidate is timed on the kernel alone, its
 output must equal the default shape's bit for bit (only the mapping of
 cells to threads changes), and the fastest is installed through
-``wf_set_launch_shape``.  Shapes are read when a launch is issued, so tune
+``wf_set_launch_shape``; where the library's own form wins nothing is.  Shapes are read when a launch is issued, so tune
 before building the solvers that should use them.
 
 Results can be cached as JSON (``save``; one file holds all three tables)
@@ -207,14 +209,37 @@ def _time_fn(fn, reps):
     return a.elapsed_time(b) / reps * 1e3  # us
 
 
+def _time_graph(fn, reps):
+    """us of fn's launches replayed from a graph (the form a step runs them in;
+    from the host a small kernel's time is the launch's)."""
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        fn()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g, stream=s):
+            fn()
+        t = min(_time_fn(g.replay, reps) for _ in range(3))
+    torch.cuda.current_stream().wait_stream(s)
+    return t
+
+
+def _rows_by_default(n):
+    """Sizes whose FP64 split half-sweep runs by rows without a shape set."""
+    return n >= 104 and (n < 144 or n % 4 != 0)
+
+
 def tune_shapes(sizes=(80,), conv=CONV_SHAPES, split=SPLIT_SHAPES, reps=10, device="cuda:0"):
     """Time every candidate shape of the convection pass (the three
     components, one launch each) and, for sizes whose finest level relaxes
-    on the split copy (FP64, n >= 80, even), of the split half-sweep (12
-    half-sweeps: a 12-sweep relax less a 6-sweep one).  Install the fastest
+    on the split copy (n >= 64, even), of the FP64 split half-sweep (12
+    half-sweeps: a 12-sweep relax less a 6-sweep one, in a graph).  The
+    library's default is a candidate of both.  Install the fastest
     per size and return {"conv": {n: rec}, "split": {n: rec}}, rec =
-    {"best": [a, b, c], "us": {"axbxc": time}}.  Raises if a shape changes
-    a result."""
+    {"best": [a, b, c], "us": {"axbxc": time}}; a split record has "default":
+    whether the library's own form won, which is then left in force (its time
+    stands under the shape that form reports).  Raises if a shape changes a
+    result."""
     from .ensemble import cavity_case
     from .solver import FlowSolver
     out = {"conv": {}, "split": {}}
@@ -228,8 +253,10 @@ def tune_shapes(sizes=(80,), conv=CONV_SHAPES, split=SPLIT_SHAPES, reps=10, devi
             for comp in range(3):
                 _abi.call("wf_conv", ctypes.byref(sol.case), comp, 0.5, dtp, stream)
 
+        set_shape("conv", n, 0, 0, 0)
+        own = shape("conv", n)
         times, ref = {}, None
-        for a, b, c in conv:
+        for a, b, c in conv if own in conv else (*conv, own):
             set_shape("conv", n, a, b, c)
             t = _time_fn(conv_pass, reps)
             got = [sol.f[k].numpy() for k in ("ustar", "vstar", "wstar")]
@@ -247,12 +274,12 @@ def tune_shapes(sizes=(80,), conv=CONV_SHAPES, split=SPLIT_SHAPES, reps=10, devi
 
         mg = sol.mg
         lev = mg.levels[0]
-        if n >= 80 and n % 2 == 0 and split:
+        if n >= 64 and n % 2 == 0 and split:
             rhs = np.random.default_rng(n).standard_normal(lev.shape)
             lev.rhs.assign(rhs)
             times, ref = {}, None
-            for c, r, _ in split:
-                set_shape("split", n, c, r)
+            for c, r, one in ((0, 0, 0), *split):   # 0: the library's own form
+                set_shape("split", n, c, r, one)
                 lev.phi.zero_()
                 mg._relax(0, 6)
                 got = lev.phi.numpy()
@@ -262,13 +289,20 @@ def tune_shapes(sizes=(80,), conv=CONV_SHAPES, split=SPLIT_SHAPES, reps=10, devi
                     set_shape("split", n, 0, 0, 0)
                     raise RuntimeError("k_rbgs_split shape %dx%d changed the result at n=%d"
                                        % (c, r, n))
-                t12 = _time_fn(lambda: mg._relax(0, 12), reps)
-                t6 = _time_fn(lambda: mg._relax(0, 6), reps)
-                times["%dx%dx1" % (c, r)] = (t12 - t6) / 12
+                t12 = _time_graph(lambda: mg._relax(0, 12), reps)
+                t6 = _time_graph(lambda: mg._relax(0, 6), reps)
+                times["%dx%dx%d" % (c, r, one)] = (t12 - t6) / 12
+            own = times.pop("0x0x0")
             best = min(times, key=times.get)
+            won = own <= times[best]
+            if won:
+                set_shape("split", n, 0, 0, 0)
+                best = "%dx%dx%d" % shape("split", n)
+                times[best] = own
             c, r, _ = (int(x) for x in best.split("x"))
-            set_shape("split", n, c, r)
-            out["split"][n] = {"best": [c, r, 1],
+            if not won:
+                set_shape("split", n, c, r)
+            out["split"][n] = {"best": [c, r, 1], "default": won, "default_us": round(own, 3),
                                "us": {k: round(v, 3) for k, v in times.items()}}
         sol.close()
     return out
@@ -283,12 +317,15 @@ def save(table, path, buckets=None, shapes=None):
     if shapes is not None:
         doc["shapes"] = {kind: {str(n): rec for n, rec in recs.items()}
                          for kind, recs in shapes.items()}
+        doc["split_forms"] = 1   # the split records know of the other forms
     with open(path, "w") as fh:
         json.dump(doc, fh, indent=1)
 
 
 def load_and_apply(path, fp32_buckets=True):
-    """Install a cached JSON table; returns the document."""
+    """Install a cached JSON table; returns the document.  Split shapes of a
+    table that was tuned before the half-sweep had other forms than rows are
+    installed only at sizes that run by rows."""
     with open(path) as fh:
         doc = json.load(fh)
     sections = ("coarse", "buckets", "shapes")
@@ -301,5 +338,9 @@ def load_and_apply(path, fp32_buckets=True):
         set_bucket_cap(int(n), rec["cap"], fp32_buckets)
     for kind, recs in doc.get("shapes", {}).items():
         for n, rec in recs.items():
-            set_shape(kind, int(n), *rec["best"])
+            if kind == "split" and (rec.get("default") or not (
+                    "split_forms" in doc or _rows_by_default(int(n)))):
+                set_shape(kind, int(n), 0, 0, 0)
+            else:
+                set_shape(kind, int(n), *rec["best"])
     return doc
