@@ -11,6 +11,8 @@
  *   - Multigrid level l >= 1 arrays are (n_l+2)^3, n_l = n >> l, one ring.
  *     Level 0 has no arrays of its own: it reads `su` and solves into `pp`
  *     in place.  Element type is double, or float when `mg_fp32` is set.
+ *   - Fields, mg_cop and mg_cop_part start on 16-byte boundaries; the other
+ *     buffers need no more than their element's alignment.
  *   - All memory is allocated and owned by the caller.  Nothing here calls
  *     cudaMalloc / cudaFree on the step path.  Only the step context keeps
  *     CUDA graph handles.
@@ -120,7 +122,8 @@ typedef struct wf_case {
                                      enough sweeps, as a polynomial of the sweep map (equal
                                      to rounding), else sweep by sweep.  WF_MG_COP_SWEEPS =
                                      sweep by sweep always */
-  void* mg_cop_part;              /* this case's scratch for it (N/2 elements) */
+  void* mg_cop_part;              /* this case's scratch for it (scratch_elems of
+                                     wf_mg_coarse_op_elems) */
 } wf_case;
 
 /* ---- library ---------------------------------------------------------- */
@@ -181,8 +184,8 @@ WF_API int wf_mg_level_elems(int32_t n, int32_t nlev, int32_t level, int64_t* el
  * the latency-bound sweeps; the results agree to rounding.  Coarsest edges
  * 4, 8, 12, 16, 20, 24 and n_coarse >= 2 only (WF_EUNSUPPORTED /
  * WF_EINVAL).  The operator is read-only once built and can be shared by
- * cases of the same size and spacing; each case needs its own scratch of
- * N/2 elements (c->mg_cop_part).  wf_mg_coarse_op_elems gives both element
+ * cases of the same size and spacing; each case needs a scratch of its own
+ * (c->mg_cop_part).  wf_mg_coarse_op_elems gives both element
  * counts (they depend on which spacings are equal). */
 WF_API int wf_mg_coarse_op_elems(const wf_case* c, int64_t* op_elems, int64_t* scratch_elems);
 WF_API int wf_mg_build_coarse_op(const wf_case* c, void* stream);

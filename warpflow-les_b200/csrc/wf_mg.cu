@@ -57,8 +57,8 @@ constexpr int LV_PP = 16, LV_SPLIT = 32;
 // The row-parity-split copies of a level in its scratch of 2 (n+2)^3 elements.
 // Both start at an odd element, because a colour's real cells of a row start at
 // an odd element of the copy (for n a multiple of 4): they are then aligned for
-// loads of two.  The last element of the copy of phi shares its place with the
-// first ones of the copy of rhs; all of these are edges of the ring, which
+// loads of two.  The last two elements of the copy of phi share their place with
+// the first two of the copy of rhs; all of these are edges of the ring, which
 // nothing reads from a level that has an rhs ring.
 template <class T>
 __host__ __device__ __forceinline__ T* split_phi(T* tmp) { return tmp + 1; }
@@ -2606,7 +2606,8 @@ static int split_in(const Lvl<T>& L, bool with_rhs, cudaStream_t s, bool first =
 //  - From 144, for n a multiple of 4, pairs marching through planes: loads of
 //    two, three of seven operands from the planes before, the next plane on its
 //    way.  rows / pairs, FP64: 128^3 4.87 / 5.46, 160^3 11.6 / 9.2, 192^3 20.6 /
-//    17.7, 256^3 40.9 / 40.0 (5.0 TB/s of DRAM traffic), 320^3 106 / 78; FP32:
+//    17.7, 256^3 40.9 / 40.0 (the 201 MB of 1.5 words a cell at 5.0 TB/s; 183.7 MB
+//    of DRAM traffic, 4.6 TB/s), 320^3 106 / 78; FP32:
 //    128^3 4.4 / 4.6, 160^3 10.4 / 7.2, 192^3 20.0 / 10.6, 256^3 35.0 / 24.2,
 //    320^3 106 / 47.  From 176 every second half-sweep runs its planes backward
 //    (what the one before touched last is still in L2: 256^3 FP64 41.5 -> 40.0).

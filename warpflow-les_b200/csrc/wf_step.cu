@@ -323,10 +323,11 @@ static bool same_bucket(const wf_case& a, const wf_case& b) {
 // should fit in about half the L2 (64 MB), so the half-sweeps, which
 // dominate a step, keep the bucket's level resident across launches.
 // Measured on B200 with 13 equal mixed-precision cases per size, one bucket
-// against a branch per case (ms per ensemble step): 32^3 1.07 vs 1.84,
-// 48^3 2.45 vs 3.29, 64^3 3.88 vs 4.44, 80^3 8.49 vs 8.94, 96^3 12.49 vs
-// 12.61.  wf_set_bucket_cap overrides the rule per size (the autotuner's
-// measurement).
+// against a branch per case (ms per ensemble step): 16^3 0.35 vs 0.52, 32^3
+// 0.81 vs 0.88, 48^3 1.94 vs 1.83, 64^3 3.38 vs 2.54, 80^3 6.3 vs 4.8, 96^3 8.5
+// vs 7.0 (1.07 vs 1.84 and 3.88 vs 4.44 at 32^3 and 64^3 before branches had
+// their chained launches, which a bucket does without).  wf_set_bucket_cap
+// overrides the rule per size (the autotuner's measurement).
 static constexpr int BUCKET_MAX_N = 1024;
 static int g_bucket_cap[2][BUCKET_MAX_N + 1];
 
@@ -614,7 +615,8 @@ int wf_ensemble_create(const wf_case* cases, int32_t ncases, int32_t mode, wf_en
   if (!cases || !out || ncases < 1) return fail(WF_EINVAL, "null argument or no cases");
   *out = nullptr;
   if (mode & ~(WF_STEP_SERIAL | WF_ENS_BUCKETS | WF_STEP_CHAIN))
-    return fail(WF_EINVAL, "ensemble mode: 0, WF_STEP_SERIAL and/or WF_ENS_BUCKETS");
+    return fail(WF_EINVAL, "ensemble mode: 0, WF_STEP_SERIAL, WF_STEP_CHAIN and/or "
+                           "WF_ENS_BUCKETS");
   for (int i = 0; i < ncases; ++i) WF_TRY(validate_case(cases[i]));
   for (int i = 0; i < ncases; ++i) prepare_fills(cases[i].n);
   PdlOff guard((mode & WF_STEP_SERIAL) != 0, (mode & WF_STEP_CHAIN) != 0);

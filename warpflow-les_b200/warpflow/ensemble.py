@@ -74,11 +74,12 @@ class Ensemble:
     kernel serves all its cases (``WF_ENS_BUCKETS``); without it every case
     is a branch of its own.  ``buckets="auto"`` (default) buckets when all
     cases have the same size and numerics, else gives each case a branch.
-    Measured on B200: 13 equal cases per size step 1.1-1.7x faster bucketed
-    (32^3 1.07 vs 1.84 ms, 96^3 12.5 vs 12.6 ms), while the 64-case mix of
-    sizes 32..96 steps 15 % faster with a branch per case (24.8 vs 28.5 ms
-    with every size bucketed): independent branches of different lengths
-    overlap one another, a bucket waits for its cases at every launch.  Once
+    Measured on B200, ms per step of 13 equal mixed-precision cases, bucketed
+    against a branch per case: 16^3 0.35 / 0.52, 32^3 0.81 / 0.88, 48^3 1.94 /
+    1.83, 64^3 3.4 / 2.5, 80^3 6.3 / 4.8, 96^3 8.5 / 7.0: from 48^3
+    ``buckets=False`` is the faster form.  A mix of sizes is faster with a
+    branch per case: independent branches of different lengths overlap one
+    another, a bucket waits for its cases at every launch.  Once
     a case has retired, or for a subset, the cases' own graphs are launched
     on a pool of ``nstreams`` streams instead.
     """
@@ -100,8 +101,8 @@ class Ensemble:
         if single_graph and len(self.solvers) > 1:
             arr = (_abi.WfCase * len(self.solvers))(*[sv.case for sv in self.solvers])
             self._graph = ctypes.c_void_p()
-            # a bucket's half-sweeps read the case table first, so they have
-            # nothing to do ahead of their wait
+            # the half-sweeps of a bucket read the case table first, so they
+            # have nothing to do ahead of their wait (its fills would)
             mode = STEP_SERIAL | (ENS_BUCKETS if self.buckets else STEP_CHAIN)
             _abi.call("wf_ensemble_create", arr, len(self.solvers), mode,
                       ctypes.byref(self._graph))
